@@ -72,9 +72,8 @@ __device__ __forceinline__ void soft_bins(const SoftHist& sh, T q, F f) {
 }
 
 template <class T, class C>
-__device__ __forceinline__ T step_len(const C& c, T E, uint64_t elec, int64_t k) {
-    const uint4 r = philox(make_uint4((uint32_t)k, (uint32_t)elec, (uint32_t)(elec >> 32), c.sim_id), c.key0,
-                           c.key1);
+__device__ __forceinline__ T step_len(const C& c, T E, const ElecRng& g, int64_t k) {
+    const uint4 r = philox_event(g, (uint32_t)k, event_words(c));
     return -Ops<T>::ln_step_word(r.y) * Ops<T>::div((T)1, sig_ruth<T>(c, E));
 }
 
@@ -132,6 +131,7 @@ __global__ void __launch_bounds__(256) k_adj_fwd(const SimConst<T> cp, const Sof
     uint32_t st = 0;
     Lane<T> L;
     uint64_t i = 0;
+    ElecRng rng{0u, 0u, 0u};
     bool have = false;
     int kstar = -1, mstar = 0;   // exit event; events up to the deepest point
     T zbest = (T)0;
@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(256) k_adj_fwd(const SimConst<T> cp, const Sof
             if (!have && j < end) {
                 i = j;
                 lane_init(L, c);
+                rng = elec_rng(c, c.first + i);
                 kstar = -1;
                 mstar = 0;
                 zbest = (T)0;
@@ -181,7 +182,7 @@ __global__ void __launch_bounds__(256) k_adj_fwd(const SimConst<T> cp, const Sof
             }
         }
         EventOut<T> ev;
-        cont_event<T, false>(L, c, c.first + i, &ev);
+        cont_event<T, false>(L, c, rng, &ev);
         if (L.outcome == MCD_OUT_BKS) kstar = (int)(L.step - 1);
         if (L.max_z > zbest) {
             zbest = L.max_z;
@@ -246,7 +247,7 @@ struct DepthAdj {
 
 // Segment m of electron i's depth sweep (the segments run last to first).
 template <class T, class C>
-__device__ __forceinline__ void depth_segment(const C& c, const AdjBuf& buf, uint64_t i, uint64_t elec, int mstar,
+__device__ __forceinline__ void depth_segment(const C& c, const AdjBuf& buf, uint64_t i, const ElecRng& rng, int mstar,
                                               int m, T g, T ij, T ins, DepthAdj<T>& A) {
     const T* ck = static_cast<const T*>(buf.ckpt);
     const size_t n = (size_t)c.num_el;
@@ -281,12 +282,12 @@ __device__ __forceinline__ void depth_segment(const C& c, const AdjBuf& buf, uin
             aY[1][j] = L.yy;
             aY[2][j] = L.yz;
             EventOut<T> ev;
-            cont_event<T, false>(L, c, elec, &ev);
+            cont_event<T, false>(L, c, rng, &ev);
         }
         for (int j = len - 1; j >= 0; --j) {   // reverse sweep
             const T E = aE[j];
             // the event's step and angles as cont_event_r computed them
-            const uint4 r = philox(event_counter((uint32_t)(k0 + j), elec, c.sim_id), c.key0, c.key1);
+            const uint4 r = philox_event(rng, (uint32_t)(k0 + j), event_words(c));
             const T s = -Ops<T>::ln_step_word(r.y) * Ops<T>::div((T)1, sig_ruth<T>(c, E));
             const T a_r = Ops<T>::div(c.a0, E);
             const T s2 = Ops<T>::div(a_r * Ops<T>::unit(r.z), a_r + Ops<T>::unit_c(r.z));
@@ -418,6 +419,7 @@ __global__ void __launch_bounds__(128, 8) k_adj_bwd(const SimConst<T> cp, const 
     // lane state: its electron, the exit event, the segment to sweep next and
     // (exit energy) the adjoint of E and the electron's parameter sums
     int64_t cur = -1;
+    ElecRng rng{0u, 0u, 0u};
     int ks = 0, m = 0;
     T lam = (T)0, sj = (T)0, sn = (T)0;
     DepthAdj<T> dA{};   // depth: the adjoints carried between segments
@@ -428,6 +430,7 @@ __global__ void __launch_bounds__(128, 8) k_adj_bwd(const SimConst<T> cp, const 
             const int64_t e = bks_take(f, buf, idle, lane);
             if (e >= 0) {
                 cur = e;
+                rng = elec_rng(c, c.first + (uint64_t)e);
                 ks = buf.kstar[e];
                 m = (ks - 1) / kSeg;
                 // the sweep runs in the transport precision: lambda is a
@@ -440,9 +443,8 @@ __global__ void __launch_bounds__(128, 8) k_adj_bwd(const SimConst<T> cp, const 
         if (__ballot_sync(0xffffffffu, cur >= 0) == 0u) break;
         if (cur < 0) continue;
         const uint64_t i = (uint64_t)cur;
-        const uint64_t elec = c.first + i;
         if constexpr (DEPTH) {   // one segment per trip; lam holds g = dL/dZ
-            depth_segment<T>(c, buf, i, elec, ks, m, lam, ij, ins, dA);
+            depth_segment<T>(c, buf, i, rng, ks, m, lam, ij, ins, dA);
             if (--m < 0) {
                 gj += dA.sj;
                 gn += dA.sn;
@@ -456,7 +458,7 @@ __global__ void __launch_bounds__(128, 8) k_adj_bwd(const SimConst<T> cp, const 
         T Eseg[kSeg], sseg[kSeg];
         T E = ck[(size_t)m * n + i];
         for (int j = 0; j < len; ++j) {   // recompute the segment exactly as the forward did
-            const T s = step_len<T>(c, E, elec, k0 + j);
+            const T s = step_len<T>(c, E, rng, k0 + j);
             Eseg[j] = E;
             sseg[j] = s;
             E = E - Ops<T>::mul_rn(s, stopping<T>(c, E));
@@ -506,7 +508,7 @@ __global__ void __launch_bounds__(256) k_adj_chain(const SimConst<T> cp, const S
     if (i < (uint64_t)c.num_el) {
         const int kstar = buf.kstar[i];
         if (kstar >= 0) {
-            const uint64_t elec = c.first + i;
+            const ElecRng rng = elec_rng(c, c.first + i);
             T Ed;
             if (sh.quantity == MCD_ADJ_MAX_DEPTH) {
                 // the forward's own events up to the deepest point
@@ -514,13 +516,13 @@ __global__ void __launch_bounds__(256) k_adj_chain(const SimConst<T> cp, const S
                 lane_init(L, c);
                 for (int k = 0; k < kstar; ++k) {
                     EventOut<T> ev;
-                    cont_event<T, false>(L, c, elec, &ev);
+                    cont_event<T, false>(L, c, rng, &ev);
                 }
                 Ed = L.z;
             } else {
                 T E = c.E0;
                 for (int k = 0; k < kstar; ++k) {
-                    const T s = step_len<T>(c, E, elec, k);
+                    const T s = step_len<T>(c, E, rng, k);
                     E = E - Ops<T>::mul_rn(s, stopping<T>(c, E));
                 }
                 Ed = E;

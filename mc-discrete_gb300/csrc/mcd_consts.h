@@ -46,6 +46,10 @@ constexpr double kPiEfour = 6.51408491409531e-14;  // cm^2 eV^2 (parameters.py:7
 constexpr double kBohrR = 5.29177210544e-11;       // m (CODATA 2022)
 constexpr double kPi = 3.141592653589793;
 
+// Philox4x32 key increments and multipliers (Salmon et al., SC'11)
+constexpr uint32_t kPhiloxW0 = 0x9E3779B9u, kPhiloxW1 = 0xBB67AE85u;
+constexpr uint32_t kPhiloxM0 = 0xD2511F53u, kPhiloxM1 = 0xCD9E8D57u;
+
 struct TableDev {
     const float* Es;
     const float* Ws;
@@ -60,11 +64,13 @@ struct TableDev {
 
 template <class T>
 struct __align__(16) SimConst {
-    // the words every event reads first, as one 16-byte load: Philox
-    // counter word 3, the key, and the events before 'long' (at most
-    // 2^32 - 1, the counter word's range)
-    uint32_t sim_id;
-    uint32_t key0, key1;
+    // the words every event reads first, as one 16-byte load: Philox counter
+    // word 3 with the key it meets in round 1 (sim id ^ key 1), the key of
+    // round 3 (both words two increments on; rounds 1 and 2 take theirs from
+    // the electron's constants, ElecRng), and the events before 'long' (at
+    // most 2^32 - 1, the counter word's range)
+    uint32_t simk;
+    uint32_t key0_3, key1_3;
     uint32_t max_scatt;
     // transport
     T E0, Emin, thickness;
@@ -261,9 +267,10 @@ inline SimConst<T> make_consts(const mcd_sim& s, const mcd_material& m,
     c.bethe = s.bethe_model;
     c.quirks = s.quirks;
     c.tally_flags = s.tally_flags;
-    c.sim_id = s.sim_id;
-    c.key0 = (uint32_t)(s.seed & 0xffffffffull);
-    c.key1 = (uint32_t)(s.seed >> 32);
+    const uint32_t key0 = (uint32_t)(s.seed & 0xffffffffull), key1 = (uint32_t)(s.seed >> 32);
+    c.simk = s.sim_id ^ key1;
+    c.key0_3 = key0 + 2u * kPhiloxW0;
+    c.key1_3 = key1 + 2u * kPhiloxW1;
     c.max_scatt = (s.max_scatt > 0 && s.max_scatt < (int64_t)UINT32_MAX) ? (uint32_t)s.max_scatt : UINT32_MAX;
     c.first = s.first_electron;
     c.num_el = s.num_el;

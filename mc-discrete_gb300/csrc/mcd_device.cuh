@@ -17,18 +17,62 @@ namespace mcd {
 // electron lo, electron hi, sim id), key = seed: every (sim, electron, event)
 // has its own block of four 32-bit words, so any electron range can be
 // re-run, sharded or recomputed (the adjoint) without stored state.
+//
+// Rounds 1 and 2 meet the electron's words with the constant key, so what
+// depends on them alone is computed once per electron (ElecRng): the round-1
+// product of word 2, which fixes words 0 and 1 entering round 2, and the
+// round-2 product of word 0.  An event then issues 18 of the 20 wide
+// products.  The three constants replace the electron's index in a lane's
+// registers, which is recovered from them when the electron ends (the
+// multipliers are odd, so their low products are invertible).
+// Measured: 64-simulation batch 77.4 -> 75.7 ms, exit-energy forward and
+// backward with its host calls 3.18 -> 3.01 ms (depth 1.87 -> 1.77 ms).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ uint4 philox(uint4 c, uint32_t k0, uint32_t k1) {
+__host__ __device__ constexpr uint32_t inv32(uint32_t a) {   // a^-1 mod 2^32, a odd (Newton)
+    uint32_t x = a;
+    for (int i = 0; i < 5; ++i) x *= 2u - a * x;
+    return x;
+}
+
+struct ElecRng {
+    uint32_t b;   // word 1 entering round 2 ^ the round-2 key 0
+    uint32_t d;   // high product of round 2's word 0 ^ the round-2 key 1
+    uint32_t e;   // its low product: word 3 entering round 3
+};
+
+template <class C>
+__device__ __forceinline__ ElecRng elec_rng(const C& c, uint64_t elec) {
+    const uint32_t k0 = c.key0_3 - 2u * kPhiloxW0;
+    const uint64_t p1 = (uint64_t)kPhiloxM1 * (uint32_t)(elec >> 32);
+    const uint64_t p0 = (uint64_t)kPhiloxM0 * ((uint32_t)(p1 >> 32) ^ (uint32_t)elec ^ k0);
+    return ElecRng{(uint32_t)p1 ^ (c.key0_3 - kPhiloxW0), (uint32_t)(p0 >> 32) ^ (c.key1_3 - kPhiloxW1), (uint32_t)p0};
+}
+
+// the electron index elec_rng was given
+template <class C>
+__device__ __forceinline__ uint64_t elec_index(const C& c, const ElecRng& g) {
+    const uint32_t k0 = c.key0_3 - 2u * kPhiloxW0;
+    const uint32_t hi = (g.b ^ (c.key0_3 - kPhiloxW0)) * inv32(kPhiloxM1);
+    const uint32_t lo = (g.e * inv32(kPhiloxM0)) ^ k0 ^ (uint32_t)(((uint64_t)kPhiloxM1 * hi) >> 32);
+    return ((uint64_t)hi << 32) | lo;
+}
+
+// the four words of event `step`; w = the constant block's first words
+__device__ __forceinline__ uint4 philox_event(const ElecRng& g, uint32_t step, const uint4 w) {
+    const uint64_t p0 = (uint64_t)kPhiloxM0 * step;                              // round 1
+    const uint64_t p1 = (uint64_t)kPhiloxM1 * ((uint32_t)(p0 >> 32) ^ w.x);      // round 2
+    uint4 c = make_uint4((uint32_t)(p1 >> 32) ^ g.b, (uint32_t)p1, g.d ^ (uint32_t)p0, g.e);
+    uint32_t k0 = w.y, k1 = w.z;
 #pragma unroll
-    for (int r = 0; r < 10; ++r) {
-        if (r) {
-            k0 += 0x9E3779B9u;
-            k1 += 0xBB67AE85u;
+    for (int r = 2; r < 10; ++r) {
+        if (r > 2) {
+            k0 += kPhiloxW0;
+            k1 += kPhiloxW1;
         }
         // one 32 x 32 -> 64-bit product per multiplier
-        const uint64_t p0 = (uint64_t)0xD2511F53u * c.x;
-        const uint64_t p1 = (uint64_t)0xCD9E8D57u * c.z;
-        c = make_uint4((uint32_t)(p1 >> 32) ^ c.y ^ k0, (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c.w ^ k1, (uint32_t)p0);
+        const uint64_t q0 = (uint64_t)kPhiloxM0 * c.x;
+        const uint64_t q1 = (uint64_t)kPhiloxM1 * c.z;
+        c = make_uint4((uint32_t)(q1 >> 32) ^ c.y ^ k0, (uint32_t)q1, (uint32_t)(q0 >> 32) ^ c.w ^ k1, (uint32_t)q0);
     }
     return c;
 }
@@ -417,7 +461,7 @@ struct Lane {
     uint32_t step;   // events so far (Philox counter word 0)
     uint32_t outcome;
     uint32_t flags;
-    uint32_t nan_n, clamp_n, lpath_n;
+    uint32_t odd_n;   // NaN-angle events (DS) or long steps (continuous)
 };
 
 template <class T, class C>
@@ -435,7 +479,7 @@ __device__ __forceinline__ void lane_init(Lane<T>& L, const C& c) {
     L.step = 0;
     L.outcome = MCD_OUT_NONE;
     L.flags = 0;
-    L.nan_n = L.clamp_n = L.lpath_n = 0;
+    L.odd_n = 0;
 }
 
 // One event's record, filled when a ring is attached.
@@ -664,10 +708,6 @@ __device__ __forceinline__ T ruth_s2(const C& c, T E, uint32_t u) {
     }
 }
 
-__device__ __forceinline__ uint4 event_counter(uint32_t step, uint64_t elec, uint32_t sim_id) {
-    return make_uint4(step, (uint32_t)elec, (uint32_t)(elec >> 32), sim_id);
-}
-
 // One DS event from its four random words r (the step counter already
 // advanced).  Returns the channel code.
 template <class T, bool REC, class C>
@@ -765,7 +805,7 @@ __device__ __forceinline__ int ds_event_r(Lane<T>& L, const C& c, const uint4 r,
             s2 = (T)0.5 * Ops<T>::div(q, (T)1 + Ops<T>::sqrt_((T)1 - q));
         } else {
             L.flags |= F_NAN;
-            L.nan_n += 1;
+            L.odd_n += 1;
             s2 = (c.bits & MCD_Q_NAN_DIRECTION) ? Ops<T>::nan_() : (T)0;
         }
     }
@@ -793,15 +833,15 @@ __device__ __forceinline__ int ds_event_r(Lane<T>& L, const C& c, const uint4 r,
     return ch;
 }
 
-// sim_id, key0, key1, max_scatt in one load: the 'long' check that opens
+// simk, key0_3, key1_3, max_scatt in one load: the 'long' check that opens
 // every event (MC/tools/singleScatter.py:19-23) and its Philox block
 template <class C>
 __device__ __forceinline__ uint4 event_words(const C& c) {
-    return *reinterpret_cast<const uint4*>(&c.sim_id);
+    return *reinterpret_cast<const uint4*>(&c.simk);
 }
 
 template <class T, bool REC, class C>
-__device__ __forceinline__ int ds_event(Lane<T>& L, const C& c, uint64_t elec, EventOut<T>* ev,
+__device__ __forceinline__ int ds_event(Lane<T>& L, const C& c, const ElecRng& g, EventOut<T>* ev,
                                         bool use_tab = false) {
     const uint4 w = event_words(c);
     if (L.step >= w.w) {
@@ -809,7 +849,7 @@ __device__ __forceinline__ int ds_event(Lane<T>& L, const C& c, uint64_t elec, E
         L.E_row = L.E;
         return -1;
     }
-    const uint4 r = philox(event_counter(L.step, elec, w.x), w.y, w.z);
+    const uint4 r = philox_event(g, L.step, w);
     L.step += 1;
     return ds_event_r<T, REC>(L, c, r, ev, use_tab);
 }
@@ -825,16 +865,15 @@ __device__ __forceinline__ int cont_event_r(Lane<T>& L, const C& c, const uint4 
     const T s = -Ops<T>::ln_step_word(r.y) * Ops<T>::div((T)1, sR);
     if (!(s < (T)1e4)) {
         L.flags |= F_LONG_PATH;
-        L.lpath_n += 1;
+        L.odd_n += 1;
     }
     const T x0 = L.x, y0 = L.y, z0 = L.z;
     lane_move(L, c, s);
     // a product that is never fused into the energy update, so that the
     // adjoint's recomputation reproduces these energies bit for bit
     T dE = Ops<T>::mul_rn(s, stopping<T>(c, E));
-    if (!(dE < E)) {
+    if (!(dE < E)) {   // ends the electron (E - dE = 0), so once at most
         L.flags |= F_CLAMPED;
-        L.clamp_n += 1;
         dE = E;
     }
     // the two-division form: in this event the single-division one of
@@ -863,14 +902,14 @@ __device__ __forceinline__ int cont_event_r(Lane<T>& L, const C& c, const uint4 
 }
 
 template <class T, bool REC, class C>
-__device__ __forceinline__ int cont_event(Lane<T>& L, const C& c, uint64_t elec, EventOut<T>* ev) {
+__device__ __forceinline__ int cont_event(Lane<T>& L, const C& c, const ElecRng& g, EventOut<T>* ev) {
     const uint4 w = event_words(c);
     if (L.step >= w.w) {
         L.outcome = MCD_OUT_LONG;
         L.E_row = L.E;
         return -1;
     }
-    const uint4 r = philox(event_counter(L.step, elec, w.x), w.y, w.z);
+    const uint4 r = philox_event(g, L.step, w);
     L.step += 1;
     return cont_event_r<T, REC>(L, c, r, ev);
 }

@@ -73,9 +73,8 @@ __device__ __forceinline__ uint32_t finish_electron(const C& c, const Lane<T>& L
     atomicAdd(&bt.events, (unsigned long long)L.step);
     atomicAdd(&bt.sum_steps2, (double)L.step * (double)L.step);
     if (L.flags & F_DOUBLE_ROW) atomicAdd(&bt.double_rows, 1u);
-    if (L.nan_n) atomicAdd(&bt.nan_events, L.nan_n);
-    if (L.clamp_n) atomicAdd(&bt.clamped, L.clamp_n);
-    if (L.lpath_n) atomicAdd(&bt.long_path, L.lpath_n);
+    if (L.odd_n) atomicAdd((c.bits & kBitCont) ? &bt.long_path : &bt.nan_events, L.odd_n);
+    if (L.flags & F_CLAMPED) atomicAdd(&bt.clamped, 1u);
     if (L.flags & F_TABLE_RANGE) atomicAdd(&bt.table_range, 1u);
     if (L.outcome == MCD_OUT_BKS) {
         const double e = (double)L.E_row;
@@ -146,12 +145,12 @@ __global__ void __launch_bounds__(256) k_plain(const SimConst<T> cp, mcd_tally* 
     if (i < (uint64_t)c.num_el) {
         Lane<T> L;
         lane_init(L, c);
-        const uint64_t elec = c.first + i;
+        const ElecRng rng = elec_rng(c, c.first + i);
         const bool chan = (c.tally_flags & MCD_TALLY_CHANNELS) != 0;
         while (L.outcome == MCD_OUT_NONE) {
             EventOut<T> ev;
-            const int ch = (MODE == MCD_MODE_DS) ? ds_event<T, REC>(L, c, elec, &ev, c.sig != nullptr)
-                                                 : cont_event<T, REC>(L, c, elec, &ev);
+            const int ch = (MODE == MCD_MODE_DS) ? ds_event<T, REC>(L, c, rng, &ev, c.sig != nullptr)
+                                                 : cont_event<T, REC>(L, c, rng, &ev);
             if (ch >= 0) {
                 if (REC) st |= ring_append(ring, (uint32_t)i, L.step, ev);
                 if (chan) atomicAdd(&bt.channel[ch], 1ull);
@@ -301,7 +300,7 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
     const unsigned lt = (1u << lane) - 1u;
     Lane<float> L;
     int sim = 0;
-    uint64_t elec = 0;
+    ElecRng rng{0u, 0u, 0u};
     bool have = false;
     bool exhausted = false;
     uint32_t st = 0;
@@ -323,7 +322,7 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
                         if (s_pre[mid] <= g) lo = mid; else hi = mid;
                     }
                     sim = s_perm[lo];
-                    elec = s_c[sim].first + (g - s_pre[lo]);   // the Philox electron index
+                    rng = elec_rng(s_c[sim], s_c[sim].first + (g - s_pre[lo]));
                     lane_init(L, s_c[sim]);
                     have = true;
                 }
@@ -340,15 +339,15 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
             EventOut<float> ev;
             int ch;
             if (!(c.bits & kBitCont))
-                ch = ds_event<float, REC>(L, c, elec, &ev, !inline_sigma && c.sig != nullptr);
+                ch = ds_event<float, REC>(L, c, rng, &ev, !inline_sigma && c.sig != nullptr);
             else
-                ch = cont_event<float, REC>(L, c, elec, &ev);
-            if (REC && ch >= 0) st |= ring_append(ring, (uint32_t)(elec - c.first), L.step, ev);
+                ch = cont_event<float, REC>(L, c, rng, &ev);
+            if (REC && ch >= 0) st |= ring_append(ring, (uint32_t)(elec_index(c, rng) - c.first), L.step, ev);
             if (ch >= 0 && (c.bits & kBitChan)) atomicAdd(&s_t[sim].channel[ch], 1ull);
             if (L.outcome != MCD_OUT_NONE) {
                 const mcd_electron_out& r = rows[sim];
                 const ElOut eo{r.outcome, r.flags, r.final_E, r.dir, r.last_pos, r.max_z, r.n_events};
-                st |= finish_electron(c, L, elec - c.first, s_t[sim], tallies + sim, eo);
+                st |= finish_electron(c, L, elec_index(c, rng) - c.first, s_t[sim], tallies + sim, eo);
                 have = false;
             }
         }
@@ -530,15 +529,15 @@ __global__ void __launch_bounds__(32) k_plain_lanes64(const SimConst<double> cp,
     const int lane = threadIdx.x & 31, t = lane & 15, h = lane >> 4;
     const uint64_t i = (uint64_t)blockIdx.x * 2 + (uint64_t)h;
     bool active = i < (uint64_t)c.num_el;
-    const uint64_t elec = c.first + i;
-    const uint4 w = event_words(c);   // sim id, Philox key, event limit
+    const ElecRng rng = elec_rng(c, c.first + i);
+    const uint4 w = event_words(c);   // sim id and Philox key words, event limit
     const bool chan = (c.tally_flags & MCD_TALLY_CHANNELS) != 0;
     Lane<double> L;
     lane_init(L, c);
     uint32_t base = 0, pz = 0;
     EventPre<double> mine{};
     auto ahead = [&]() {   // lane t: the event at step base + t
-        const uint4 r = philox(event_counter(base + (uint32_t)t, elec, w.x), w.y, w.z);
+        const uint4 r = philox_event(rng, base + (uint32_t)t, w);
         pz = r.z;
         mine.ln_y = ln_word(r.y);
         azimuth<double>(c, r.w, &mine.cph, &mine.sph);
