@@ -20,6 +20,12 @@ namespace mcd {
 
 // Per-block sums; the per-event counters (events, channels) are 64-bit, as
 // one persistent block can see more than 2^32 events of a channel.
+// Channel counts (MCD_TALLY_CHANNELS): every event of an electron has one
+// channel, so only the others are counted event by event and Rutherford's
+// count is the rest of `events` at the flush.  Counting it per event too put
+// up to 32 lanes of every warp on one 64-bit shared counter, a serialised
+// compare-and-swap loop: six uneven simulations (5.5e7 events) took 17.5 ms
+// for it, 9.4 ms without.
 struct BlockTally {
     unsigned int outcome[8];
     unsigned int double_rows, nan_events, clamped, long_path, table_range, pad_;
@@ -38,7 +44,7 @@ __device__ __forceinline__ void add_u64(unsigned long long* p, unsigned long lon
     if (v) atomicAdd(p, v);
 }
 
-__device__ __forceinline__ void bt_flush(const BlockTally& t, mcd_tally* g) {
+__device__ __forceinline__ void bt_flush(const BlockTally& t, mcd_tally* g, bool chan) {
     // called by one thread per simulation
     bool any = t.events != 0;
     for (int k = 0; k < 8; ++k) any |= t.outcome[k] != 0;
@@ -50,7 +56,14 @@ __device__ __forceinline__ void bt_flush(const BlockTally& t, mcd_tally* g) {
     add_u64(&g->clamped, t.clamped);
     add_u64(&g->long_path, t.long_path);
     add_u64(&g->table_range, t.table_range);
-    for (int k = 0; k < MCD_MAX_CHANNELS; ++k) add_u64(&g->channel[k], t.channel[k]);
+    if (chan) {
+        unsigned long long others = 0;
+        for (int k = 1; k < MCD_MAX_CHANNELS; ++k) {
+            others += t.channel[k];
+            add_u64(&g->channel[k], t.channel[k]);
+        }
+        add_u64(&g->channel[MCD_CH_RUTH], t.events - others);
+    }
     if (t.sum_E != 0.0) atomicAdd(&g->sum_E_bks, t.sum_E);
     if (t.sum_E2 != 0.0) atomicAdd(&g->sum_E2_bks, t.sum_E2);
     if (t.sum_steps2 != 0.0) atomicAdd(&g->sum_steps2, t.sum_steps2);
@@ -153,14 +166,14 @@ __global__ void __launch_bounds__(256) k_plain(const SimConst<T> cp, mcd_tally* 
                                                  : cont_event<T, REC>(L, c, rng, &ev);
             if (ch >= 0) {
                 if (REC) st |= ring_append(ring, (uint32_t)i, L.step, ev);
-                if (chan) atomicAdd(&bt.channel[ch], 1ull);
+                if (chan && ch != MCD_CH_RUTH) atomicAdd(&bt.channel[ch], 1ull);
             }
         }
         st |= finish_electron(c, L, i, bt, tally, eo);
     }
     or_status(status, st);
     __syncthreads();
-    if (threadIdx.x == 0) bt_flush(bt, tally);
+    if (threadIdx.x == 0) bt_flush(bt, tally, (c.bits & kBitChan) != 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -170,7 +183,8 @@ struct BatchHeader {
     unsigned long long queue;   // next electron to hand out
     unsigned long long total;   // electrons over all simulations
     int32_t nsims;
-    int32_t pad_[11];
+    int32_t chan;               // some simulation counts channels
+    int32_t pad_[10];
 };
 
 constexpr int kBatchMaxSims = 256;
@@ -244,7 +258,7 @@ static void batch_order(const mcd_sim* sims, int nsims, int32_t* perm) {
     }
 }
 
-template <bool REC>
+template <bool REC, bool CHAN>
 __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, int refill, uint32_t* status,
                                              const mcd_event_ring& ring, int inline_sigma);
 
@@ -254,22 +268,27 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
 // constant blocks in shared memory): on the 64-simulation workload the
 // second, in blocks of 576, is 1.2% faster (78.2 against 79.1 ms); five
 // blocks of 256 at 48 registers were 26% slower.
-// REC: append every event to the ring.
+// REC: append every event to the ring.  The event loop exists twice, CHAN
+// for batches in which some simulation counts channels, so that the others
+// test nothing per event (one test there cost 1% of the 64 simulations); the
+// counts of members that do not ask are dropped at the flush.
 template <bool REC = false>
 __global__ void __launch_bounds__(1024) k_batched(uint8_t* ws, mcd_tally* tallies, int refill,
                                                   uint32_t* status, const mcd_event_ring ring = mcd_event_ring{},
                                                   int inline_sigma = 0) {
-    batched_body<REC>(ws, tallies, refill, status, ring, inline_sigma);
+    if (reinterpret_cast<const BatchHeader*>(ws)->chan) batched_body<REC, true>(ws, tallies, refill, status, ring, inline_sigma);
+    else batched_body<REC, false>(ws, tallies, refill, status, ring, inline_sigma);
 }
 
 template <bool REC = false>
 __global__ void __launch_bounds__(576, 2) k_batched_lr(uint8_t* ws, mcd_tally* tallies, int refill,
                                                        uint32_t* status, const mcd_event_ring ring = mcd_event_ring{},
                                                        int inline_sigma = 0) {
-    batched_body<REC>(ws, tallies, refill, status, ring, inline_sigma);
+    if (reinterpret_cast<const BatchHeader*>(ws)->chan) batched_body<REC, true>(ws, tallies, refill, status, ring, inline_sigma);
+    else batched_body<REC, false>(ws, tallies, refill, status, ring, inline_sigma);
 }
 
-template <bool REC>
+template <bool REC, bool CHAN>
 __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, int refill, uint32_t* status,
                                              const mcd_event_ring& ring, int inline_sigma) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -343,7 +362,7 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
             else
                 ch = cont_event<float, REC>(L, c, rng, &ev);
             if (REC && ch >= 0) st |= ring_append(ring, (uint32_t)(elec_index(c, rng) - c.first), L.step, ev);
-            if (ch >= 0 && (c.bits & kBitChan)) atomicAdd(&s_t[sim].channel[ch], 1ull);
+            if (CHAN && ch > MCD_CH_RUTH) atomicAdd(&s_t[sim].channel[ch], 1ull);
             if (L.outcome != MCD_OUT_NONE) {
                 const mcd_electron_out& r = rows[sim];
                 const ElOut eo{r.outcome, r.flags, r.final_E, r.dir, r.last_pos, r.max_z, r.n_events};
@@ -354,7 +373,8 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
     }
     or_status(status, st);
     __syncthreads();
-    for (int k = threadIdx.x; k < nsims; k += blockDim.x) bt_flush(s_t[k], tallies + k);
+    for (int k = threadIdx.x; k < nsims; k += blockDim.x)
+        bt_flush(s_t[k], tallies + k, (s_c[k].bits & kBitChan) != 0);
 }
 
 // Cross-section tables of a prepared batch: one thread per (table slot, grid
@@ -569,7 +589,7 @@ __global__ void __launch_bounds__(32) k_plain_lanes64(const SimConst<double> cp,
             L.step += 1;
             EventOut<double> ev;
             const int ch = ds_event_r<double, false>(L, c, make_uint4(0u, 0u, rz, 0u), &ev, c.sig != nullptr, &pre);
-            if (chan && t == 0 && ch >= 0) atomicAdd(&bt.channel[ch], 1ull);
+            if (chan && t == 0 && ch > MCD_CH_RUTH) atomicAdd(&bt.channel[ch], 1ull);
         }
         if (L.outcome != MCD_OUT_NONE) {
             if (t == 0) st |= finish_electron(c, L, i, bt, tally, eo);
@@ -578,7 +598,7 @@ __global__ void __launch_bounds__(32) k_plain_lanes64(const SimConst<double> cp,
     }
     or_status(status, st);
     __syncthreads();
-    if (threadIdx.x == 0) bt_flush(bt, tally);
+    if (threadIdx.x == 0) bt_flush(bt, tally, chan);
 }
 
 static int launch_lanes64(const SimConst<double>& c, mcd_tally* tally, const ElOut& eo, uint32_t* status,
@@ -759,6 +779,7 @@ extern "C" int mcd_batch_prepare(const mcd_sim* sims, int32_t nsims, const mcd_m
     h->queue = 0;
     h->total = acc;
     h->nsims = nsims;
+    for (int k = 0; k < nsims; ++k) h->chan |= (sims[k].tally_flags & MCD_TALLY_CHANNELS) ? 1 : 0;
     if (rc == MCD_OK) {
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         const unsigned grid = (unsigned)(((long long)nsims * kSigRowsMax + 255) / 256);
@@ -968,6 +989,7 @@ extern "C" int mcd_run_batched_noalloc(const mcd_sim* sims, int32_t nsims, const
     h->queue = 0;
     h->total = acc;
     h->nsims = nsims;
+    for (int k = 0; k < nsims; ++k) h->chan |= (sims[k].tally_flags & MCD_TALLY_CHANNELS) ? 1 : 0;
     pack_rows(sims, nsims, host);
     // the core only: cross sections come from the callers' tables or are
     // evaluated inline
