@@ -310,13 +310,12 @@ int mcd_build_sigma_table(const mcd_sim* sim, const mcd_material* mat,
  * mode only (gryz = the outermost shell's table, which samples every
  * Gryzinski loss, MC/tools/scattering.py:625).  electrons and ring may be
  * NULL.  tally and status are device pointers.  block_size is 1, 2, 4, 8,
- * 16 or a multiple of 32 up to 256, or 0: 128, halved down to 8 while the
- * grid would leave SMs idle, so that a small job spreads over more SMs with
- * fewer lanes each, and for FP64 transport further down to 2 while the grid
- * stays within one warp per scheduler; there an FP64 DS run without a ring
- * puts two electrons on each warp, one per half-warp whose lanes compute
- * the coming events' random numbers and the functions of them that do not
- * depend on the trajectory (results do not depend on any of this).  A DS
+ * 16 or a multiple of 32 up to 256, or 0: a run of few electrons per SM takes
+ * 8, 16 or 32 lanes of a warp per electron, which share the work that is not
+ * on the trajectory's chain; a larger one a thread per electron in blocks of
+ * 128, halved down to 8 while the grid would leave SMs idle (FP64: down to 2
+ * while it stays within one warp per scheduler).  Results do not depend on
+ * any of this.  A DS
  * simulation with a sigma_table reads its channel cross sections from it.  */
 int mcd_run(const mcd_sim* sim, const mcd_material* mat,
             const mcd_table* moller, const mcd_table* gryz,

@@ -403,8 +403,12 @@ __device__ __forceinline__ int table_row(const TableDev& t, T E, bool* out_of_ra
     return hi;
 }
 
+struct TableSpan {
+    int row;      // the first E row >= E
+    int lo, hi;   // the draw's column lies in [lo, hi]
+};
 template <class T>
-__device__ __forceinline__ T table_pick(const TableDev& t, T E, T U, bool* oor) {
+__device__ __forceinline__ TableSpan table_span(const TableDev& t, T E, T U, bool* oor) {
     const int ncol = t.nW - 1;
     const int kq = (int)(U * (T)MCD_GUIDE);
     int i = -1, lo = 0, hi = 0;
@@ -438,7 +442,14 @@ __device__ __forceinline__ T table_pick(const TableDev& t, T E, T U, bool* oor) 
             hi = ncol;   // masked entries (0) act as +inf
         }
     }
-    const float* row = t.cdf + (size_t)i * ncol;
+    return TableSpan{i, lo, hi};
+}
+
+template <class T>
+__device__ __forceinline__ T table_pick(const TableDev& t, T E, T U, bool* oor) {
+    const TableSpan sp = table_span<T>(t, E, U, oor);
+    int lo = sp.lo, hi = sp.hi;
+    const float* row = t.cdf + (size_t)sp.row * (t.nW - 1);
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
         const float v = __ldg(row + mid);
@@ -450,8 +461,7 @@ __device__ __forceinline__ T table_pick(const TableDev& t, T E, T U, bool* oor) 
 // ---------------------------------------------------------------------------
 // electron state
 // ---------------------------------------------------------------------------
-enum : uint32_t { F_DOUBLE_ROW = 1u, F_NAN = 2u, F_TABLE_RANGE = 4u, F_CLAMPED = 8u, F_LONG_PATH = 16u,
-                  F_DIFFRACTING = 32u };
+enum : uint32_t { F_DOUBLE_ROW = 1u, F_NAN = 2u, F_TABLE_RANGE = 4u, F_CLAMPED = 8u, F_LONG_PATH = 16u };
 
 template <class T>
 struct Lane {
@@ -482,6 +492,13 @@ __device__ __forceinline__ void lane_init(Lane<T>& L, const C& c) {
     L.odd_n = 0;
 }
 
+// An electron that reaches the event limit ends there.
+template <class T>
+__device__ __forceinline__ void lane_long(Lane<T>& L) {
+    L.outcome = MCD_OUT_LONG;
+    L.E_row = L.E;
+}
+
 // One event's record, filled when a ring is attached.
 template <class T>
 struct EventOut {
@@ -493,13 +510,13 @@ struct EventOut {
 // Position update and the exit tests (MC/tools/electron.py:64-84): leaving
 // through the bottom face on a diffraction event's step is 'trdf'.
 template <class T, class C>
-__device__ __forceinline__ void lane_move(Lane<T>& L, const C& c, T s) {
+__device__ __forceinline__ void lane_move(Lane<T>& L, const C& c, T s, bool diffracting = false) {
     const T nz = L.z + s * L.dz;
     if (nz <= (T)0) {
         L.outcome = MCD_OUT_BKS;
         L.E_row = L.E;
     } else if ((c.bits & kBitFilm) && nz >= c.thickness) {
-        L.outcome = (L.flags & F_DIFFRACTING) ? MCD_OUT_TRDF : MCD_OUT_TRSM;
+        L.outcome = diffracting ? MCD_OUT_TRDF : MCD_OUT_TRSM;
         L.E_row = L.E;
     } else {
         L.x += s * L.dx;
@@ -598,14 +615,24 @@ __device__ __forceinline__ void lane_rotate(Lane<T>& L, const C& c, T s2, uint32
 // Channel and E times the total inverse mean free path from the tabulated
 // cumulative cross sections: linear interpolation in log2(E) between two rows
 // of E * (running sum); the comparison with U * E * total needs no division.
+struct SigRow {
+    const float* r0;   // the row below E; the next one is sig_S floats on
+    float f;           // E's place between them
+};
 template <class C>
-__device__ __forceinline__ int tab_pick(const C& c, float E, float U, float* Etot_out) {
+__device__ __forceinline__ SigRow sig_row_at(const C& c, float E) {
     float t = fmaf(__log2f(E), c.sig_inv, c.sig_off);
     t = fminf(fmaxf(t, 0.0f), c.sig_tmax);
     const int i = (int)t;
-    const float f = t - (float)i;
+    return SigRow{static_cast<const float*>(c.sig) + i * bits_S(c), t - (float)i};
+}
+
+template <class C>
+__device__ __forceinline__ int tab_pick(const C& c, float E, float U, float* Etot_out) {
+    const SigRow row = sig_row_at(c, E);
+    const float f = row.f;
     const int S = bits_S(c);
-    const float* r0 = static_cast<const float*>(c.sig) + i * S;
+    const float* r0 = row.r0;
     const float* r1 = r0 + S;
     const int K = bits_K(c);
     // column 0 holds the total, columns 1.. the running sums before it
@@ -650,21 +677,33 @@ __device__ __forceinline__ int tab_pick(const C& c, float E, float U, float* Eto
 // compared with the fractions of the other channels.  Returns -1 for a cell
 // whose nodes straddle a channel threshold (its flag is set): the caller
 // evaluates the cross sections.
+struct Sig64Cell {
+    const double* r;
+    double f;   // E's place in the cell
+    __device__ __forceinline__ bool smooth() const { return __ldg(reinterpret_cast<const long long*>(r)) == 0ll; }
+    __device__ __forceinline__ double at(int col) const {
+        const double2 lo = __ldg(reinterpret_cast<const double2*>(r + 2 + 4 * col));
+        const double2 hi = __ldg(reinterpret_cast<const double2*>(r + 4 + 4 * col));
+        return fma(fma(fma(hi.y, f, hi.x), f, lo.y), f, lo.x);
+    }
+};
 template <class C>
-__device__ __forceinline__ int tab_pick64(const C& c, double E, double U, double* mfp_out) {
+__device__ __forceinline__ Sig64Cell sig64_cell(const C& c, double E) {
     const long long b = __double_as_longlong(E);   // E > 0
     int blk = (int)(b >> 52) - 1023 - (int)c.sig_l0;
     blk = blk < 0 ? 0 : (blk > c.sig_rows - 1 ? c.sig_rows - 1 : blk);
     const int i = (int)(b >> 44) & (kSig64Cells - 1);
-    const double f = __longlong_as_double(((b << 8) & 0x000fffffffffff00ll) | 0x3ff0000000000000ll) - 1.0;
+    return Sig64Cell{static_cast<const double*>(c.sig) +
+                         ((size_t)blk * kSig64Cells + i) * sig64_stride(bits_K(c)),
+                     __longlong_as_double(((b << 8) & 0x000fffffffffff00ll) | 0x3ff0000000000000ll) - 1.0};
+}
+
+template <class C>
+__device__ __forceinline__ int tab_pick64(const C& c, double E, double U, double* mfp_out) {
     const int K = bits_K(c);
-    const double* r = static_cast<const double*>(c.sig) + ((size_t)blk * kSig64Cells + i) * sig64_stride(K);
-    if (__ldg(reinterpret_cast<const long long*>(r)) != 0ll) return -1;
-    auto at = [&](int col) {
-        const double2 lo = __ldg(reinterpret_cast<const double2*>(r + 2 + 4 * col));
-        const double2 hi = __ldg(reinterpret_cast<const double2*>(r + 4 + 4 * col));
-        return fma(fma(fma(hi.y, f, hi.x), f, lo.y), f, lo.x);
-    };
+    const Sig64Cell cell = sig64_cell(c, E);
+    if (!cell.smooth()) return -1;
+    auto at = [&](int col) { return cell.at(col); };
     double mfp = at(0);
     double u = U;
     if (c.bits & kBitDiff) {
@@ -690,40 +729,49 @@ __device__ __forceinline__ int tab_pick64(const C& c, double E, double U, double
 // The trajectory-independent functions of an event's Philox words, when
 // another lane has computed them ahead: ln U of the step's uniform, the
 // azimuth's cos and sin (with the half-phi fold applied), the channel
-// pick's uniform, and the Rutherford angle's a0 U and 1 - U.
+// pick's uniform, and the polar angle's a0 U (DS; U in continuous mode) and
+// 1 - U; the two words the W tables' draw and an event record still need.
 template <class T>
-struct EventPre {
+struct __align__(16) EventPre {
     T ln_y, cph, sph, ux, a0u, uzc;
+    uint32_t rz, rw;
 };
+
 
 // Rutherford sin^2(theta/2) = a U / (a + 1 - U), a = a0 / E
 // (MC/tools/scattering.py:125-152); for the DS event in FP32 with one
 // division as a0 U / (a0 + E (1 - U)).
 template <class T, class C>
-__device__ __forceinline__ T ruth_s2(const C& c, T E, uint32_t u) {
-    if constexpr (sizeof(T) == 4) {
-        return Ops<T>::div(c.a0 * Ops<T>::unit(u), fmaf(E, Ops<T>::unit_c(u), c.a0));
-    } else {
-        return c.a0 * Ops<T>::unit(u) * rcp_pos(fma(E, Ops<T>::unit_c(u), c.a0));
+__device__ __forceinline__ T ruth_s2(const C& c, T E, T a0u, T uzc) {
+    if constexpr (sizeof(T) == 4) return Ops<T>::div(a0u, fmaf(E, uzc, c.a0));
+    else return a0u * rcp_pos(fma(E, uzc, c.a0));
+}
+
+// sin^2(theta/2) of a binary collision that loses W
+// (MC/tools/scattering.py:156-179)
+template <class T, class C>
+__device__ __forceinline__ T collide(Lane<T>& L, const C& c, T E, T W) {
+    if (W <= (E - c.Ef) * (T)0.5) {
+        const T q = Ops<T>::div(W, E);
+        return (T)0.5 * Ops<T>::div(q, (T)1 + Ops<T>::sqrt_((T)1 - q));
     }
+    L.flags |= F_NAN;
+    L.odd_n += 1;
+    return (c.bits & MCD_Q_NAN_DIRECTION) ? Ops<T>::nan_() : (T)0;
 }
 
 // One DS event from its four random words r (the step counter already
 // advanced).  Returns the channel code.
 template <class T, bool REC, class C>
 __device__ __forceinline__ int ds_event_r(Lane<T>& L, const C& c, const uint4 r, EventOut<T>* ev,
-                                          bool use_tab = false, const EventPre<T>* pre = nullptr) {
+                                          bool use_tab = false) {
     const T E = L.E;
     int ch = MCD_CH_QUINN;
     T inv_tot;
     // FP64: the azimuth's cos/sin depend on the word alone; computed first,
-    // their FP64 chain overlaps the channel pick's instead of closing the
-    // event (or given, computed ahead by another lane)
+    // their FP64 chain overlaps the channel pick's instead of closing the event
     T cph = (T)0, sph = (T)0;
-    if constexpr (sizeof(T) == 8) {
-        if (pre) cph = pre->cph, sph = pre->sph;
-        else azimuth<T>(c, r.w, &cph, &sph);
-    }
+    if constexpr (sizeof(T) == 8) azimuth<T>(c, r.w, &cph, &sph);
     if (use_tab) {
         if constexpr (sizeof(T) == 4) {
             float Etot;
@@ -731,7 +779,7 @@ __device__ __forceinline__ int ds_event_r(Lane<T>& L, const C& c, const uint4 r,
             inv_tot = Ops<T>::div(E, (T)Etot);
         } else {
             double mfp;
-            ch = tab_pick64(c, E, pre ? pre->ux : Ops<T>::unit(r.x), &mfp);
+            ch = tab_pick64(c, E, Ops<T>::unit(r.x), &mfp);
             if (ch >= 0) inv_tot = mfp;
             else use_tab = false, ch = MCD_CH_QUINN;   // a threshold inside the cell
         }
@@ -753,7 +801,7 @@ __device__ __forceinline__ int ds_event_r(Lane<T>& L, const C& c, const uint4 r,
         const T cumQ = tot;
         if (c.bits & kBitDiff) tot += c.dS;
         // --- channel (MC/tools/scattering.py:39-59)
-        const T target = (pre ? pre->ux : Ops<T>::unit(r.x)) * tot;
+        const T target = Ops<T>::unit(r.x) * tot;
         T cum = sR;
         if (target <= cum) {
             ch = MCD_CH_RUTH;
@@ -773,21 +821,16 @@ __device__ __forceinline__ int ds_event_r(Lane<T>& L, const C& c, const uint4 r,
         inv_tot = Ops<T>::div((T)1, tot);
     }
     // --- path length (MC/tools/scattering.py:540-565): a diffraction event
-    // steps with mean free path xip_g and marks the electron diffracting
+    // steps with mean free path xip_g, and leaves as 'trdf' through the bottom
     const bool diff_ev = ch == MCD_CH_DIFF;
-    L.flags = diff_ev ? (L.flags | F_DIFFRACTING) : (L.flags & ~F_DIFFRACTING);
-    const T s = -(pre ? pre->ln_y : Ops<T>::ln_step_word(r.y)) * (diff_ev ? c.xip : inv_tot);
+    const T s = -Ops<T>::ln_step_word(r.y) * (diff_ev ? c.xip : inv_tot);
     const T x0 = L.x, y0 = L.y, z0 = L.z;
-    lane_move(L, c, s);
+    lane_move(L, c, s, diff_ev);
     // --- energy loss and polar angle (MC/tools/scattering.py:568-679)
     T W, s2;
     if (ch == MCD_CH_RUTH) {
         W = (T)0;
-        if constexpr (sizeof(T) == 8) {
-            s2 = pre ? pre->a0u * rcp_pos(fma(E, pre->uzc, c.a0)) : ruth_s2<T>(c, E, r.z);
-        } else {
-            s2 = ruth_s2<T>(c, E, r.z);
-        }
+        s2 = ruth_s2<T>(c, E, c.a0 * Ops<T>::unit(r.z), Ops<T>::unit_c(r.z));
     } else if (ch == MCD_CH_QUINN) {
         W = c.Epl;
         s2 = (T)0;
@@ -799,15 +842,7 @@ __device__ __forceinline__ int ds_event_r(Lane<T>& L, const C& c, const uint4 r,
         bool oor = false;
         W = table_pick<T>(c.tab[ch != MCD_CH_MOLLER], E, Ops<T>::unit(r.z), &oor);
         if (oor) L.flags |= F_TABLE_RANGE;
-        // binary collision (MC/tools/scattering.py:156-179)
-        if (W <= (E - c.Ef) * (T)0.5) {
-            const T q = Ops<T>::div(W, E);
-            s2 = (T)0.5 * Ops<T>::div(q, (T)1 + Ops<T>::sqrt_((T)1 - q));
-        } else {
-            L.flags |= F_NAN;
-            L.odd_n += 1;
-            s2 = (c.bits & MCD_Q_NAN_DIRECTION) ? Ops<T>::nan_() : (T)0;
-        }
+        s2 = collide(L, c, E, W);
     }
     const T uphi = Ops<T>::unit(r.w);
     if (REC) {
@@ -845,8 +880,7 @@ __device__ __forceinline__ int ds_event(Lane<T>& L, const C& c, const ElecRng& g
                                         bool use_tab = false) {
     const uint4 w = event_words(c);
     if (L.step >= w.w) {
-        L.outcome = MCD_OUT_LONG;
-        L.E_row = L.E;
+        lane_long(L);
         return -1;
     }
     const uint4 r = philox_event(g, L.step, w);
@@ -859,10 +893,11 @@ __device__ __forceinline__ int ds_event(Lane<T>& L, const C& c, const ElecRng& g
 // MC/tools/singleScatter.py:210-239, with the Bethe law the mode names)
 // ---------------------------------------------------------------------------
 template <class T, bool REC, class C>
-__device__ __forceinline__ int cont_event_r(Lane<T>& L, const C& c, const uint4 r, EventOut<T>* ev) {
+__device__ __forceinline__ int cont_event_r(Lane<T>& L, const C& c, const uint4 r, EventOut<T>* ev,
+                                            const EventPre<T>* pre = nullptr) {
     const T E = L.E;
     const T sR = sig_ruth<T>(c, E);
-    const T s = -Ops<T>::ln_step_word(r.y) * Ops<T>::div((T)1, sR);
+    const T s = -(pre ? pre->ln_y : Ops<T>::ln_step_word(r.y)) * Ops<T>::div((T)1, sR);
     if (!(s < (T)1e4)) {
         L.flags |= F_LONG_PATH;
         L.odd_n += 1;
@@ -879,7 +914,7 @@ __device__ __forceinline__ int cont_event_r(Lane<T>& L, const C& c, const uint4 
     // the two-division form: in this event the single-division one of
     // ruth_s2 measured 1% slower
     const T a = Ops<T>::div(c.a0, E);
-    const T s2 = Ops<T>::div(a * Ops<T>::unit(r.z), a + Ops<T>::unit_c(r.z));
+    const T s2 = Ops<T>::div(a * (pre ? pre->a0u : Ops<T>::unit(r.z)), a + (pre ? pre->uzc : Ops<T>::unit_c(r.z)));
     const T uphi = Ops<T>::unit(r.w);
     if (REC) {
         ev->s2 = s2;
@@ -897,16 +932,32 @@ __device__ __forceinline__ int cont_event_r(Lane<T>& L, const C& c, const uint4 
     }
     const bool left = L.outcome != MCD_OUT_NONE;
     if (!left || (c.bits & MCD_Q_CROSSING_STEP)) lane_lose(L, c, dE);
-    if (L.outcome == MCD_OUT_NONE) lane_rotate(L, c, s2, r.w);
+    if (L.outcome == MCD_OUT_NONE) {
+        if (pre) lane_rotate_cs(L, s2, pre->cph, pre->sph);
+        else lane_rotate(L, c, s2, r.w);
+    }
     return MCD_CH_RUTH;
+}
+
+// The values an event computes from its words r alone
+template <class T, int MODE, class C>
+__device__ __forceinline__ EventPre<T> event_pre(const C& c, const uint4 r) {
+    EventPre<T> p;
+    p.ln_y = Ops<T>::ln_step_word(r.y);
+    azimuth<T>(c, r.w, &p.cph, &p.sph);
+    p.ux = Ops<T>::unit(r.x);
+    p.a0u = MODE == MCD_MODE_DS ? c.a0 * Ops<T>::unit(r.z) : Ops<T>::unit(r.z);
+    p.uzc = Ops<T>::unit_c(r.z);
+    p.rz = r.z;
+    p.rw = r.w;
+    return p;
 }
 
 template <class T, bool REC, class C>
 __device__ __forceinline__ int cont_event(Lane<T>& L, const C& c, const ElecRng& g, EventOut<T>* ev) {
     const uint4 w = event_words(c);
     if (L.step >= w.w) {
-        L.outcome = MCD_OUT_LONG;
-        L.E_row = L.E;
+        lane_long(L);
         return -1;
     }
     const uint4 r = philox_event(g, L.step, w);

@@ -2,6 +2,7 @@
 //
 //  k_plain    one thread per electron, one launch per simulation
 //             (replaces multiTraj_DS/_cont, MC/tools/multiScatter.py:66-229)
+//             (small runs: several lanes per electron, mcd_lanes.cu)
 //  k_batched  persistent grid over many simulations; a global queue hands
 //             out electrons and a warp takes new ones as soon as `refill` of
 //             its lanes are idle, so uneven trajectory lengths do not idle
@@ -14,128 +15,10 @@
 #include <stdint.h>
 #include <string.h>
 
-#include "mcd_device.cuh"
+#include "mcd_lanes.h"
+#include "mcd_tally.cuh"
 
 namespace mcd {
-
-// Per-block sums; the per-event counters (events, channels) are 64-bit, as
-// one persistent block can see more than 2^32 events of a channel.
-// Channel counts (MCD_TALLY_CHANNELS): every event of an electron has one
-// channel, so only the others are counted event by event and Rutherford's
-// count is the rest of `events` at the flush.  Counting it per event too put
-// up to 32 lanes of every warp on one 64-bit shared counter, a serialised
-// compare-and-swap loop: six uneven simulations (5.5e7 events) took 17.5 ms
-// for it, 9.4 ms without.
-struct BlockTally {
-    unsigned int outcome[8];
-    unsigned int double_rows, nan_events, clamped, long_path, table_range, pad_;
-    unsigned long long events;
-    double sum_E, sum_E2, sum_steps2;
-    unsigned long long channel[MCD_MAX_CHANNELS];
-};
-
-__device__ __forceinline__ void bt_zero(BlockTally* t, int n) {
-    unsigned int* p = reinterpret_cast<unsigned int*>(t);
-    const int words = n * (int)(sizeof(BlockTally) / 4);
-    for (int i = threadIdx.x; i < words; i += blockDim.x) p[i] = 0u;
-}
-
-__device__ __forceinline__ void add_u64(unsigned long long* p, unsigned long long v) {
-    if (v) atomicAdd(p, v);
-}
-
-__device__ __forceinline__ void bt_flush(const BlockTally& t, mcd_tally* g, bool chan) {
-    // called by one thread per simulation
-    bool any = t.events != 0;
-    for (int k = 0; k < 8; ++k) any |= t.outcome[k] != 0;
-    if (!any) return;
-    for (int k = 0; k < 8; ++k) add_u64(&g->outcome[k], t.outcome[k]);
-    add_u64(&g->events, t.events);
-    add_u64(&g->double_rows, t.double_rows);
-    add_u64(&g->nan_events, t.nan_events);
-    add_u64(&g->clamped, t.clamped);
-    add_u64(&g->long_path, t.long_path);
-    add_u64(&g->table_range, t.table_range);
-    if (chan) {
-        unsigned long long others = 0;
-        for (int k = 1; k < MCD_MAX_CHANNELS; ++k) {
-            others += t.channel[k];
-            add_u64(&g->channel[k], t.channel[k]);
-        }
-        add_u64(&g->channel[MCD_CH_RUTH], t.events - others);
-    }
-    if (t.sum_E != 0.0) atomicAdd(&g->sum_E_bks, t.sum_E);
-    if (t.sum_E2 != 0.0) atomicAdd(&g->sum_E2_bks, t.sum_E2);
-    if (t.sum_steps2 != 0.0) atomicAdd(&g->sum_steps2, t.sum_steps2);
-}
-
-struct ElOut {
-    uint8_t* outcome;
-    uint8_t* flags;
-    void* final_E;
-    void* dir;
-    void* last_pos;
-    void* max_z;
-    int32_t* n_events;
-};
-
-template <class T, class C>
-__device__ __forceinline__ uint32_t finish_electron(const C& c, const Lane<T>& L, uint64_t i, BlockTally& bt,
-                                                    mcd_tally* gt, const ElOut& eo) {
-    atomicAdd(&bt.outcome[L.outcome & 7], 1u);
-    atomicAdd(&bt.events, (unsigned long long)L.step);
-    atomicAdd(&bt.sum_steps2, (double)L.step * (double)L.step);
-    if (L.flags & F_DOUBLE_ROW) atomicAdd(&bt.double_rows, 1u);
-    if (L.odd_n) atomicAdd((c.bits & kBitCont) ? &bt.long_path : &bt.nan_events, L.odd_n);
-    if (L.flags & F_CLAMPED) atomicAdd(&bt.clamped, 1u);
-    if (L.flags & F_TABLE_RANGE) atomicAdd(&bt.table_range, 1u);
-    if (L.outcome == MCD_OUT_BKS) {
-        const double e = (double)L.E_row;
-        atomicAdd(&bt.sum_E, e);
-        atomicAdd(&bt.sum_E2, e * e);
-        if (c.hE > 0) {
-            const T f = L.E_row * c.invWE;
-            if (f >= (T)0 && f < (T)c.hE) atomicAdd(&gt->hist_E[(int)f], 1ull);
-        }
-        if (c.hT > 0) {
-            const T th = Ops<T>::acos_deg(-L.dz) * c.invWT;
-            if (th >= (T)0 && th < (T)c.hT) atomicAdd(&gt->hist_T[(int)th], 1ull);
-        }
-    }
-    if (eo.outcome) eo.outcome[i] = (uint8_t)L.outcome;
-    if (eo.flags) eo.flags[i] = (uint8_t)(L.flags & (F_DOUBLE_ROW | F_NAN));
-    const size_t n = (size_t)c.num_el;
-    if (eo.final_E) static_cast<T*>(eo.final_E)[i] = L.E_row;
-    if (eo.dir) {
-        T* d = static_cast<T*>(eo.dir);
-        d[i] = L.dx;
-        d[n + i] = L.dy;
-        d[2 * n + i] = L.dz;
-    }
-    if (eo.last_pos) {
-        T* p = static_cast<T*>(eo.last_pos);
-        p[i] = L.x;
-        p[n + i] = L.y;
-        p[2 * n + i] = L.z;
-    }
-    if (eo.max_z) static_cast<T*>(eo.max_z)[i] = L.max_z;
-    if (eo.n_events) eo.n_events[i] = (int32_t)L.step;
-    uint32_t st = 0;
-    if (L.flags & F_NAN) st |= MCD_FLAG_NAN;
-    if (L.flags & F_TABLE_RANGE) st |= MCD_FLAG_TABLE_RANGE;
-    if (L.flags & F_CLAMPED) st |= MCD_FLAG_CLAMPED;
-    if (L.flags & F_LONG_PATH) st |= MCD_FLAG_LONG_PATH;
-    if (L.outcome == MCD_OUT_LONG) st |= MCD_FLAG_LONG;
-    return st;
-}
-
-// Called by every thread of the block; a block smaller than a warp (plain
-// launches of 1 to 16 threads) leaves lanes that never exist, so the
-// reduction names the lanes present.
-__device__ __forceinline__ void or_status(uint32_t* status, uint32_t st) {
-    const uint32_t w = __reduce_or_sync(__activemask(), st);
-    if ((threadIdx.x & 31) == 0 && w) atomicOr(status, w);
-}
 
 // ---------------------------------------------------------------------------
 // plain kernel: one thread per electron
@@ -529,87 +412,6 @@ inline void share_sigma_tables(const mcd_sim* sims, int nsims, const SimConst<do
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-// FP64 DS transport of a small run, one warp per two electrons.  Such a run
-// lasts as long as its longest trajectory, one dependent chain of
-// instructions.  The 16 lanes of each half-warp run their electron's events
-// in lockstep (every lane holds the same state) and compute, 16 events
-// ahead and one event per lane, what does not depend on the trajectory: the
-// event's Philox block, ln U of its step uniform, the azimuth's cos and
-// sin, and the uniforms of the channel pick and the polar angle (the values
-// the event itself would compute); an event takes them from its lane by
-// shuffles, so the chain no longer carries them.  The trajectories are
-// k_plain's, bit for bit.
-__global__ void __launch_bounds__(32) k_plain_lanes64(const SimConst<double> cp, mcd_tally* tally, const ElOut eo,
-                                                      uint32_t* status) {
-    __shared__ BlockTally bt;
-    __shared__ SimConst<double> c;
-    if (threadIdx.x == 0) c = cp;
-    bt_zero(&bt, 1);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, t = lane & 15, h = lane >> 4;
-    const uint64_t i = (uint64_t)blockIdx.x * 2 + (uint64_t)h;
-    bool active = i < (uint64_t)c.num_el;
-    const ElecRng rng = elec_rng(c, c.first + i);
-    const uint4 w = event_words(c);   // sim id and Philox key words, event limit
-    const bool chan = (c.tally_flags & MCD_TALLY_CHANNELS) != 0;
-    Lane<double> L;
-    lane_init(L, c);
-    uint32_t base = 0, pz = 0;
-    EventPre<double> mine{};
-    auto ahead = [&]() {   // lane t: the event at step base + t
-        const uint4 r = philox_event(rng, base + (uint32_t)t, w);
-        pz = r.z;
-        mine.ln_y = ln_word(r.y);
-        azimuth<double>(c, r.w, &mine.cph, &mine.sph);
-        mine.ux = Ops<double>::unit(r.x);
-        mine.a0u = c.a0 * Ops<double>::unit(r.z);
-        mine.uzc = Ops<double>::unit_c(r.z);
-    };
-    ahead();
-    uint32_t st = 0;
-    while (__any_sync(0xffffffffu, active)) {
-        if (active && L.step - base == 16u) {
-            base += 16u;
-            ahead();
-        }
-        const int src = (h << 4) | (int)((L.step - base) & 15u);
-        const uint32_t rz = __shfl_sync(0xffffffffu, pz, src);   // the W tables' uniform (inelastic events)
-        EventPre<double> pre;
-        pre.ln_y = __shfl_sync(0xffffffffu, mine.ln_y, src);
-        pre.cph = __shfl_sync(0xffffffffu, mine.cph, src);
-        pre.sph = __shfl_sync(0xffffffffu, mine.sph, src);
-        pre.ux = __shfl_sync(0xffffffffu, mine.ux, src);
-        pre.a0u = __shfl_sync(0xffffffffu, mine.a0u, src);
-        pre.uzc = __shfl_sync(0xffffffffu, mine.uzc, src);
-        if (!active) continue;
-        if (L.step >= w.w) {   // the 'long' check that opens every event (MC/tools/singleScatter.py:19-23)
-            L.outcome = MCD_OUT_LONG;
-            L.E_row = L.E;
-        } else {
-            L.step += 1;
-            EventOut<double> ev;
-            const int ch = ds_event_r<double, false>(L, c, make_uint4(0u, 0u, rz, 0u), &ev, c.sig != nullptr, &pre);
-            if (chan && t == 0 && ch > MCD_CH_RUTH) atomicAdd(&bt.channel[ch], 1ull);
-        }
-        if (L.outcome != MCD_OUT_NONE) {
-            if (t == 0) st |= finish_electron(c, L, i, bt, tally, eo);
-            active = false;
-        }
-    }
-    or_status(status, st);
-    __syncthreads();
-    if (threadIdx.x == 0) bt_flush(bt, tally, chan);
-}
-
-static int launch_lanes64(const SimConst<double>& c, mcd_tally* tally, const ElOut& eo, uint32_t* status,
-                          cudaStream_t st) {
-    const unsigned long long grid = ((unsigned long long)c.num_el + 1) / 2;
-    if (grid == 0) return MCD_OK;
-    if (grid > 0x7fffffffull) return MCD_ETOOBIG;
-    k_plain_lanes64<<<(unsigned)grid, 32, 0, st>>>(c, tally, eo, status);
-    return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
-}
-
 template <class T, int MODE, bool REC>
 static int launch_plain(const SimConst<T>& c, int block, mcd_tally* tally, const ElOut& eo,
                         const mcd_event_ring& ring, uint32_t* status, cudaStream_t st) {
@@ -630,6 +432,35 @@ static int dispatch_plain(const SimConst<T>& c, int block, mcd_tally* tally, con
                : launch_plain<T, MCD_MODE_CONT, false>(c, block, tally, eo, ring, status, st);
 }
 
+// Lanes per electron of an automatic run (mcd_lanes.cu): 0 for a thread per
+// electron.  More lanes make an electron's chain shorter, but a warp issues
+// for fewer electrons, so the width falls as the run fills the GPU; the lines
+// (in electrons per SM) lie where the two sides measured equal on 152 SMs,
+// kernel times in ms, 0 = a thread per electron:
+//   FP32 DS (Si, table)  1000: 0.30 with 32, 0.58 with 0;  3500: 0.45 / 0.46
+//                        with 32 / 16;  5000: 0.53 / 0.55 with 16 / 8;
+//                        10000: 0.73 / 0.77 with 8 / 0;  14000: 1.05 / 0.77
+//   (Au: 10000 1.93 / 3.01 with 8 / 0, 20000 3.14 / 2.97; Cu without a table:
+//   10000 1.44 / 1.97, 14000 2.03 / 1.97)
+//   FP32 continuous      1000: 0.23 / 0.27 with 32 / 0;  2500: 0.31 / 0.28
+//   FP64 DS (Si, table)  700: 2.27 / 2.38 with 32 / 16;  1500: 2.65 / 2.66 with
+//                        16 / 8;  3500: 3.48 / 4.35 with 8 / 0;  5000: 4.96 / 4.76
+//   without a table      Si 5000: 13.3 / 14.7 with 8 / 0, 7500 19.7 / 15.3;
+//                        Au 14000: 33 / 66 (the plain kernel evaluates a
+//                        cross section per shell in every event)
+//   FP64 continuous      300: 3.69 / 3.81 with 32 / 8;  1500: 3.99 / 4.55 with 8
+//                        / 0;  2500: 4.72 / 4.54
+static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) {
+    const int64_t e = s.num_el / sms;   // electrons per SM
+    if (s.precision == MCD_FP32) {
+        if (s.mode != MCD_MODE_DS) return e < 10 ? 32 : 0;
+        return e < 23 ? 32 : e < 33 ? 16 : e < 70 ? 8 : 0;
+    }
+    if (s.mode != MCD_MODE_DS) return e < 3 ? 32 : e < 10 ? 8 : 0;
+    const int most = s.sigma_table ? 28 : 12 * (m.n_shells > 3 ? m.n_shells : 3);
+    return e < 5 ? 32 : e < 10 ? 16 : e < most ? 8 : 0;
+}
+
 }  // namespace mcd
 
 using namespace mcd;
@@ -640,23 +471,20 @@ extern "C" int mcd_run(const mcd_sim* sim, const mcd_material* mat, const mcd_ta
     if (!sim || !mat || !tally || !status) return MCD_EINVAL;
     const int rc = check_sim(*sim, *mat, moller, gryz);
     if (rc != MCD_OK) return rc;
-    const bool automatic = block_size <= 0;
-    if (automatic) {
-        // automatic: 128 threads, halved (down to 8) while the grid would
-        // leave SMs idle, so that a small job spreads over the GPU: its
-        // trajectories are latency chains, and an SM with fewer lanes runs
-        // each chain faster (1000 FP32 electrons: 1.00 ms in 32 blocks of 32,
-        // 0.82 ms in 125 blocks of 8).  FP64 goes further, down to 2 threads
-        // while the grid stays within one warp per scheduler (4 per SM):
-        // fewer lanes per warp diverge less, and the longest FP64 chain
-        // shares its scheduler with no other warp (1000 FP64 electrons with
-        // their table: 7.37 ms in blocks of 8, 6.69 ms in blocks of 2,
-        // 8.70 ms in blocks of 1, where schedulers hold two warps)
+    // automatic: a small run takes several lanes per electron (mcd_lanes.cu),
+    // a larger one a thread per electron
+    int group = 0;
+    if (block_size <= 0) {
         block_size = 128;
         int dev = 0, sms = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             return MCD_ECUDA;
+        group = lanes_per_electron(*sim, *mat, sms);
+        // a thread per electron: 128 threads, halved (down to 8) while the
+        // grid would leave SMs idle, so that a small job spreads over the GPU;
+        // FP64 further, down to 2 while the grid stays within one warp per
+        // scheduler (4 per SM): fewer lanes per warp diverge less
         while (block_size > 8 && (sim->num_el + block_size - 1) / block_size < sms) block_size /= 2;
         if (sim->precision == MCD_FP64)
             while (block_size > 2 && 2 * ((sim->num_el + block_size - 1) / block_size) <= 4ll * sms) block_size /= 2;
@@ -686,14 +514,12 @@ extern "C" int mcd_run(const mcd_sim* sim, const mcd_material* mat, const mcd_ta
     const mcd_table* tg = sim->mode == MCD_MODE_DS ? gryz : nullptr;
     if (sim->precision == MCD_FP64) {
         const SimConst<double> c = make_consts<double>(*sim, *mat, tm, tg);
-        // where the automatic size reached two electrons per warp, a DS run
-        // without an event ring puts the warp's idle lanes to work
-        if (automatic && block_size == 2 && sim->mode == MCD_MODE_DS && !rec)
-            return launch_lanes64(c, tally, eo, status, st);
+        if (group) return launch_lanes<double>(c, group, tally, eo, rg, rec, status, st);
         return dispatch_plain<double>(c, block_size, tally, eo, rg, rec, status, st);
     }
-    return dispatch_plain<float>(make_consts<float>(*sim, *mat, tm, tg), block_size, tally, eo, rg, rec, status,
-                                 st);
+    const SimConst<float> c = make_consts<float>(*sim, *mat, tm, tg);
+    if (group) return launch_lanes<float>(c, group, tally, eo, rg, rec, status, st);
+    return dispatch_plain<float>(c, block_size, tally, eo, rg, rec, status, st);
 }
 
 extern "C" size_t mcd_sigma_table_bytes(void) { return kSigTableBytes; }
