@@ -312,7 +312,9 @@ int mcd_build_sigma_table(const mcd_sim* sim, const mcd_material* mat,
  * NULL.  tally and status are device pointers.  block_size is 1, 2, 4, 8,
  * 16 or a multiple of 32 up to 256, or 0: a run of few electrons per SM takes
  * 8, 16 or 32 lanes of a warp per electron, which share the work that is not
- * on the trajectory's chain; a larger one a thread per electron in blocks of
+ * on the trajectory's chain; a larger FP32 run one resident block per SM that
+ * refills its lanes and compacts its warps (continuous mode: where the lengths
+ * of the trajectories differ); the others a thread per electron in blocks of
  * 128, halved down to 8 while the grid would leave SMs idle (FP64: down to 2
  * while it stays within one warp per scheduler).  Results do not depend on
  * any of this.  A DS
@@ -332,7 +334,9 @@ int mcd_run(const mcd_sim* sim, const mcd_material* mat,
  * per group of DS simulations with the same material, Wc and density) that
  * the kernel interpolates instead of evaluating 3 + n_shells formulas per
  * event (tune variant bit 1 keeps the formulas).
- * mcd_run_batched then only resets the queue and launches, so it can be
+ * mcd_run_batched then only resets the queue and launches (the persistent
+ * kernel, and after it the one that runs down the electrons still on their way
+ * when the queue is empty, which it lists in the workspace), so it can be
  * captured in a CUDA graph.  tallies[nsims] and status are device pointers.
  * Replaces MapScatterer.__call__ (MC/doScatter.py:54-95) with its pool of
  * multiTraj_* jobs.                                                          */

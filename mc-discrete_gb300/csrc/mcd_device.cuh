@@ -939,14 +939,15 @@ __device__ __forceinline__ int cont_event_r(Lane<T>& L, const C& c, const uint4 
     return MCD_CH_RUTH;
 }
 
-// The values an event computes from its words r alone
-template <class T, int MODE, class C>
-__device__ __forceinline__ EventPre<T> event_pre(const C& c, const uint4 r) {
+// The values an event computes from its words r alone (ang: the factor of
+// the polar angle's U, a0 in DS and 1 in continuous mode)
+template <class T, class C>
+__device__ __forceinline__ EventPre<T> event_pre(const C& c, const uint4 r, T ang) {
     EventPre<T> p;
     p.ln_y = Ops<T>::ln_step_word(r.y);
     azimuth<T>(c, r.w, &p.cph, &p.sph);
     p.ux = Ops<T>::unit(r.x);
-    p.a0u = MODE == MCD_MODE_DS ? c.a0 * Ops<T>::unit(r.z) : Ops<T>::unit(r.z);
+    p.a0u = ang * Ops<T>::unit(r.z);
     p.uzc = Ops<T>::unit_c(r.z);
     p.rz = r.z;
     p.rw = r.w;

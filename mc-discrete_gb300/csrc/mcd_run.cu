@@ -1,0 +1,66 @@
+// mcd_run.cu - one FP32 simulation of more electrons than the small-run kernel
+// takes, one resident block per SM.
+//
+// Block b runs every gridDim.x-th electron: its lanes take the next of its
+// share as they fall idle, and when the share is handed out the block runs down
+// with compaction (mcd_drain.cuh).  No queue in global memory is needed, since
+// the shares of the SMs are statistically alike.  512 threads where they hold
+// the share (more registers, less to meet at a barrier), 1024 beyond.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "mcd_drain.cuh"
+#include "mcd_run.h"
+
+namespace mcd {
+
+template <int MODE, bool REC, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_run(const SimConst<float> cp, mcd_tally* tally, const mcd_electron_out eo,
+                                                 const mcd_event_ring ring, uint32_t* status) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ BlockTally bt;
+    __shared__ SimConst<float> c;
+    __shared__ mcd_electron_out rows;
+    if (threadIdx.x == 0) {
+        c = cp;
+        rows = eo;
+    }
+    bt_zero(&bt, 1);
+    __syncthreads();
+    const OneSim<MODE> run{c, bt, tally, rows};
+    const unsigned count = (unsigned)(((unsigned long long)c.num_el - blockIdx.x + gridDim.x - 1) / gridDim.x);
+    auto take = [&](unsigned k, Lane<float>& L, ElecRng& rng, int& sim) {
+        rng = elec_rng(c, c.first + blockIdx.x + (uint64_t)k * gridDim.x);
+        lane_init(L, c);
+        sim = 0;
+    };
+    const bool chan = (c.bits & kBitChan) != 0;
+    const uint32_t st = MODE == MCD_MODE_DS && chan ? drain_run<REC, true>(run, count, take, smem, ring, false)
+                                                    : drain_run<REC, false>(run, count, take, smem, ring, false);
+    or_status(status, st);
+    __syncthreads();
+    if (threadIdx.x == 0) bt_flush(bt, tally, chan);
+}
+
+template <int MODE, bool REC>
+static int launch_threads(const SimConst<float>& c, int sms, mcd_tally* tally, const mcd_electron_out& rows,
+                          const mcd_event_ring& ring, uint32_t* status, cudaStream_t st) {
+    const unsigned grid = (unsigned)(c.num_el < sms ? c.num_el : sms);
+    if (grid == 0) return MCD_OK;
+    if (c.num_el <= (int64_t)512 * sms)
+        k_run<MODE, REC, 512><<<grid, 512, drain_smem(512), st>>>(c, tally, rows, ring, status);
+    else
+        k_run<MODE, REC, 1024><<<grid, 1024, drain_smem(1024), st>>>(c, tally, rows, ring, status);
+    return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
+}
+
+int launch_run(const SimConst<float>& c, int sms, mcd_tally* tally, const mcd_electron_out& rows,
+               const mcd_event_ring& ring, bool rec, uint32_t* status, cudaStream_t st) {
+    if (c.mode == MCD_MODE_DS)
+        return rec ? launch_threads<MCD_MODE_DS, true>(c, sms, tally, rows, ring, status, st)
+                   : launch_threads<MCD_MODE_DS, false>(c, sms, tally, rows, ring, status, st);
+    return rec ? launch_threads<MCD_MODE_CONT, true>(c, sms, tally, rows, ring, status, st)
+               : launch_threads<MCD_MODE_CONT, false>(c, sms, tally, rows, ring, status, st);
+}
+
+}  // namespace mcd

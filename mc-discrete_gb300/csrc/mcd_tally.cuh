@@ -35,7 +35,9 @@ __device__ __forceinline__ void add_u64(unsigned long long* p, unsigned long lon
 
 __device__ __forceinline__ void bt_flush(const BlockTally& t, mcd_tally* g, bool chan) {
     // called by one thread per simulation
-    bool any = t.events != 0;
+    unsigned long long others = 0;
+    for (int k = 1; chan && k < MCD_MAX_CHANNELS; ++k) others += t.channel[k];
+    bool any = t.events != 0 || others != 0;
     for (int k = 0; k < 8; ++k) any |= t.outcome[k] != 0;
     if (!any) return;
     for (int k = 0; k < 8; ++k) add_u64(&g->outcome[k], t.outcome[k]);
@@ -46,11 +48,10 @@ __device__ __forceinline__ void bt_flush(const BlockTally& t, mcd_tally* g, bool
     add_u64(&g->long_path, t.long_path);
     add_u64(&g->table_range, t.table_range);
     if (chan) {
-        unsigned long long others = 0;
-        for (int k = 1; k < MCD_MAX_CHANNELS; ++k) {
-            others += t.channel[k];
-            add_u64(&g->channel[k], t.channel[k]);
-        }
+        for (int k = 1; k < MCD_MAX_CHANNELS; ++k) add_u64(&g->channel[k], t.channel[k]);
+        // an electron's events are counted where it ends, which may be
+        // another block than ran some of them: the differences add up modulo
+        // 2^64
         add_u64(&g->channel[MCD_CH_RUTH], t.events - others);
     }
     if (t.sum_E != 0.0) atomicAdd(&g->sum_E_bks, t.sum_E);

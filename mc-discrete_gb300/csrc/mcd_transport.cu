@@ -2,7 +2,8 @@
 //
 //  k_plain    one thread per electron, one launch per simulation
 //             (replaces multiTraj_DS/_cont, MC/tools/multiScatter.py:66-229)
-//             (small runs: several lanes per electron, mcd_lanes.cu)
+//             (small runs: several lanes per electron, mcd_lanes.cu; large FP32
+//             ones: a resident block per SM, mcd_run.cu)
 //  k_batched  persistent grid over many simulations; a global queue hands
 //             out electrons and a warp takes new ones as soon as `refill` of
 //             its lanes are idle, so uneven trajectory lengths do not idle
@@ -15,8 +16,9 @@
 #include <stdint.h>
 #include <string.h>
 
+#include "mcd_drain.cuh"
 #include "mcd_lanes.h"
-#include "mcd_tally.cuh"
+#include "mcd_run.h"
 
 namespace mcd {
 
@@ -64,10 +66,11 @@ __global__ void __launch_bounds__(256) k_plain(const SimConst<T> cp, mcd_tally* 
 // ---------------------------------------------------------------------------
 struct BatchHeader {
     unsigned long long queue;   // next electron to hand out
+    unsigned long long live;    // electrons listed for the run-down kernel
     unsigned long long total;   // electrons over all simulations
     int32_t nsims;
     int32_t chan;               // some simulation counts channels
-    int32_t pad_[10];
+    int32_t pad_[8];
 };
 
 constexpr int kBatchMaxSims = 256;
@@ -109,14 +112,22 @@ __host__ __device__ constexpr size_t batch_sig_off(int nsims) {
 __host__ __device__ constexpr size_t batch_sig_bytes() {   // one table slot per simulation
     return sizeof(float) * (size_t)kSigRowsMax * kSigStride;
 }
-__host__ __device__ constexpr size_t batch_bytes(int nsims) {
+// | the electrons still on their way when the queue ran empty (seats as in
+// mcd_drain.cuh): at most one per lane of the launch
+constexpr int kLiveSeats = 1 << 18;
+__host__ __device__ constexpr size_t batch_live_off(int nsims) {
     return batch_sig_off(nsims) + batch_sig_bytes() * (size_t)nsims;
+}
+__host__ __device__ constexpr size_t batch_bytes(int nsims) {
+    return batch_live_off(nsims) + sizeof(uint32_t) * kSeatWords * (size_t)kLiveSeats;
 }
 
 __host__ __device__ constexpr size_t batch_smem(int nsims) {
     return sizeof(SimConst<float>) * nsims + sizeof(unsigned long long) * (nsims + 1) +
            sizeof(int32_t) * ((nsims + 1) & ~1) + sizeof(BlockTally) * nsims;
 }
+// ... of the run-down kernel, the drain's seats after it
+__host__ __device__ constexpr size_t batch_drain_off(int nsims) { return (batch_smem(nsims) + 15) & ~(size_t)15; }
 
 // Queue order: simulations with the longest expected trajectories first, so
 // that the last electrons handed out are short ones and the grid drains
@@ -143,7 +154,7 @@ static void batch_order(const mcd_sim* sims, int nsims, int32_t* perm) {
 
 template <bool REC, bool CHAN>
 __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, int refill, uint32_t* status,
-                                             const mcd_event_ring& ring, int inline_sigma);
+                                             const mcd_event_ring& ring, int flags);
 
 // Two register budgets of the same kernel: up to 1024 threads per block at
 // 64 registers (32 warps per SM: one block of 1024), or two blocks of up to
@@ -158,44 +169,65 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
 template <bool REC = false>
 __global__ void __launch_bounds__(1024) k_batched(uint8_t* ws, mcd_tally* tallies, int refill,
                                                   uint32_t* status, const mcd_event_ring ring = mcd_event_ring{},
-                                                  int inline_sigma = 0) {
-    if (reinterpret_cast<const BatchHeader*>(ws)->chan) batched_body<REC, true>(ws, tallies, refill, status, ring, inline_sigma);
-    else batched_body<REC, false>(ws, tallies, refill, status, ring, inline_sigma);
+                                                  int flags = 0) {
+    if (reinterpret_cast<const BatchHeader*>(ws)->chan) batched_body<REC, true>(ws, tallies, refill, status, ring, flags);
+    else batched_body<REC, false>(ws, tallies, refill, status, ring, flags);
 }
 
 template <bool REC = false>
 __global__ void __launch_bounds__(576, 2) k_batched_lr(uint8_t* ws, mcd_tally* tallies, int refill,
                                                        uint32_t* status, const mcd_event_ring ring = mcd_event_ring{},
-                                                       int inline_sigma = 0) {
-    if (reinterpret_cast<const BatchHeader*>(ws)->chan) batched_body<REC, true>(ws, tallies, refill, status, ring, inline_sigma);
-    else batched_body<REC, false>(ws, tallies, refill, status, ring, inline_sigma);
+                                                       int flags = 0) {
+    if (reinterpret_cast<const BatchHeader*>(ws)->chan) batched_body<REC, true>(ws, tallies, refill, status, ring, flags);
+    else batched_body<REC, false>(ws, tallies, refill, status, ring, flags);
 }
+
+// What a batched block keeps in shared memory: the simulations' constants,
+// queue prefix sums, order and tallies.
+struct BatchShared {
+    SimConst<float>* c;
+    unsigned long long* pre;
+    int32_t* perm;
+    BlockTally* t;
+    __device__ __forceinline__ BatchShared(uint8_t* smem, int nsims)
+        : c(reinterpret_cast<SimConst<float>*>(smem)),
+          pre(reinterpret_cast<unsigned long long*>(smem + sizeof(SimConst<float>) * nsims)),
+          perm(reinterpret_cast<int32_t*>(pre + (nsims + 1))),
+          t(reinterpret_cast<BlockTally*>(perm + ((nsims + 1) & ~1))) {}
+    __device__ __forceinline__ void load(const uint8_t* ws, int nsims) const {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(ws + batch_consts_off(nsims));
+        uint32_t* dst = reinterpret_cast<uint32_t*>(c);
+        const int words = (int)(sizeof(SimConst<float>) / 4) * nsims;
+        for (int k = threadIdx.x; k < words; k += blockDim.x) dst[k] = src[k];
+        const unsigned long long* p = reinterpret_cast<const unsigned long long*>(ws + batch_prefix_off());
+        for (int k = threadIdx.x; k <= nsims; k += blockDim.x) pre[k] = p[k];
+        const int32_t* q = reinterpret_cast<const int32_t*>(ws + batch_perm_off(nsims));
+        for (int k = threadIdx.x; k < nsims; k += blockDim.x) perm[k] = q[k];
+        bt_zero(t, nsims);
+    }
+    __device__ __forceinline__ void flush(mcd_tally* tallies, int nsims) const {
+        for (int k = threadIdx.x; k < nsims; k += blockDim.x)
+            bt_flush(t[k], tallies + k, (c[k].bits & kBitChan) != 0);
+    }
+};
+
+constexpr int kRunInline = 1;   // evaluate cross sections instead of reading the tables
+constexpr int kRunList = 2;     // list the electrons left when the queue is empty
 
 template <bool REC, bool CHAN>
 __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, int refill, uint32_t* status,
-                                             const mcd_event_ring& ring, int inline_sigma) {
+                                             const mcd_event_ring& ring, int flags) {
     extern __shared__ __align__(16) uint8_t smem[];
     BatchHeader* hdr = reinterpret_cast<BatchHeader*>(ws);
     const int nsims = hdr->nsims;
     const unsigned long long total = hdr->total;
-    SimConst<float>* s_c = reinterpret_cast<SimConst<float>*>(smem);
-    unsigned long long* s_pre = reinterpret_cast<unsigned long long*>(smem + sizeof(SimConst<float>) * nsims);
-    int32_t* s_perm = reinterpret_cast<int32_t*>(smem + sizeof(SimConst<float>) * nsims +
-                                                 sizeof(unsigned long long) * (nsims + 1));
-    BlockTally* s_t = reinterpret_cast<BlockTally*>(smem + sizeof(SimConst<float>) * nsims +
-                                                    sizeof(unsigned long long) * (nsims + 1) +
-                                                    sizeof(int32_t) * ((nsims + 1) & ~1));
-    {
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(ws + batch_consts_off(nsims));
-        uint32_t* dst = reinterpret_cast<uint32_t*>(s_c);
-        const int words = (int)(sizeof(SimConst<float>) / 4) * nsims;
-        for (int k = threadIdx.x; k < words; k += blockDim.x) dst[k] = src[k];
-        const unsigned long long* pre = reinterpret_cast<const unsigned long long*>(ws + batch_prefix_off());
-        for (int k = threadIdx.x; k <= nsims; k += blockDim.x) s_pre[k] = pre[k];
-        const int32_t* perm = reinterpret_cast<const int32_t*>(ws + batch_perm_off(nsims));
-        for (int k = threadIdx.x; k < nsims; k += blockDim.x) s_perm[k] = perm[k];
-        bt_zero(s_t, nsims);
-    }
+    const int inline_sigma = flags & kRunInline;
+    const BatchShared sh(smem, nsims);
+    SimConst<float>* s_c = sh.c;
+    unsigned long long* s_pre = sh.pre;
+    int32_t* s_perm = sh.perm;
+    BlockTally* s_t = sh.t;
+    sh.load(ws, nsims);
     __syncthreads();
 
     const int lane = threadIdx.x & 31;
@@ -229,8 +261,20 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
                     have = true;
                 }
             }
-            if (base + __popc(idle) >= total) exhausted = true;
+            // (a batch no larger than the launch is handed out in one claim per warp)
+            if (base + __popc(idle) >= total || total <= (unsigned long long)gridDim.x * blockDim.x) exhausted = true;
             idle = __ballot_sync(0xffffffffu, !have);
+            if (exhausted && (flags & kRunList)) {
+                // the run-down kernel takes the warp's electrons over
+                const unsigned busy = ~idle;
+                unsigned long long at = 0;
+                if (lane == 0 && busy) at = atomicAdd(&hdr->live, (unsigned long long)__popc(busy));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (have)
+                    seat_put(Seats{reinterpret_cast<uint32_t*>(ws + batch_live_off(nsims)), kLiveSeats},
+                             (int)at + __popc(busy & lt), L, rng, sim);
+                break;
+            }
         }
         if (idle == 0xffffffffu) {
             if (exhausted) break;
@@ -256,8 +300,35 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
     }
     or_status(status, st);
     __syncthreads();
-    for (int k = threadIdx.x; k < nsims; k += blockDim.x)
-        bt_flush(s_t[k], tallies + k, (s_c[k].bits & kBitChan) != 0);
+    sh.flush(tallies, nsims);
+}
+
+// The electrons that a batched launch listed, to their end: block b of the
+// grid takes every gridDim.x-th of them, so that each SM gets its part of
+// every simulation's.
+template <bool REC>
+__global__ void __launch_bounds__(kDrainThreads) k_rundown(uint8_t* ws, mcd_tally* tallies, uint32_t* status,
+                                                           const mcd_event_ring ring, int flags) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const BatchHeader* hdr = reinterpret_cast<const BatchHeader*>(ws);
+    const int nsims = hdr->nsims;
+    const unsigned live = (unsigned)hdr->live;
+    if (blockIdx.x >= live) return;
+    const BatchShared sh(smem, nsims);
+    sh.load(ws, nsims);
+    const ManySims run{sh.c, sh.t, tallies, reinterpret_cast<const mcd_electron_out*>(ws + batch_elout_off(nsims))};
+    const Seats list{reinterpret_cast<uint32_t*>(ws + batch_live_off(nsims)), kLiveSeats};
+    const unsigned count = (live - blockIdx.x + gridDim.x - 1) / gridDim.x;
+    auto take = [&](unsigned k, Lane<float>& L, ElecRng& rng, int& sim) {
+        seat_get(list, (int)(blockIdx.x + k * gridDim.x), L, rng, sim);
+    };
+    uint8_t* seats = smem + batch_drain_off(nsims);
+    const bool inl = (flags & kRunInline) != 0;
+    const uint32_t st = hdr->chan ? drain_run<REC, true>(run, count, take, seats, ring, inl)
+                                  : drain_run<REC, false>(run, count, take, seats, ring, inl);
+    or_status(status, st);
+    __syncthreads();
+    sh.flush(tallies, nsims);
 }
 
 // Cross-section tables of a prepared batch: one thread per (table slot, grid
@@ -461,6 +532,29 @@ static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) 
     return e < 5 ? 32 : e < 10 ? 16 : e < most ? 8 : 0;
 }
 
+// Does an automatic run of a thread per electron take one resident block per
+// SM that refills its lanes and compacts its warps (mcd_run.cu), or blocks of
+// independent threads?  The first keeps warps full where trajectory lengths
+// differ; its barriers and its own loop cost a few percent where they do not.
+// Kernel times in ms, this against independent threads:
+//   FP32 DS    from 70 electrons per SM, where the lanes of mcd_lanes.cu end
+//              (20000 electrons: Cu 1.85 / 2.00, Au 2.37 / 2.98, Si 0.74 / 0.77;
+//              40000: Cu 2.10 / 2.21, Au 2.99 / 3.36, Si 0.87 / 0.83; 1e6: Cu
+//              12.6 / 21.5, Au 14.0 / 33.4, Si 6.1 / 8.0)
+//   FP32 continuous, whose lengths differ by backscattering alone: 1e6
+//              electrons Cu 70 deg 2.64 / 4.26, Al 70 deg 1.77 / 2.27, Au 0 deg
+//              7.5 / 10.8, Cu 0 deg 3.97 / 4.30, but Al 0 deg 2.39 / 2.28; from
+//              one wave of lanes on (150000: Cu 70 deg 0.55 / 0.77; 80000:
+//              0.43 / 0.49; 40000: 0.38 / 0.36)
+static bool one_block_per_sm(const mcd_sim& s, const mcd_material& m, int sms) {
+    const int64_t e = s.num_el / sms;   // electrons per SM
+    if (s.precision != MCD_FP32 || e > INT32_MAX / 2) return false;
+    if (s.mode == MCD_MODE_DS) return e >= 70;
+    if (s.E0 < 10.0 * s.Emin) return false;   // short trajectories: the start and the end weigh more
+    if (s.s_tilt >= 60.0 || m.Z >= 40) return e >= 450;
+    return m.Z >= 25 && e >= 4000;
+}
+
 }  // namespace mcd
 
 using namespace mcd;
@@ -473,14 +567,16 @@ extern "C" int mcd_run(const mcd_sim* sim, const mcd_material* mat, const mcd_ta
     if (rc != MCD_OK) return rc;
     // automatic: a small run takes several lanes per electron (mcd_lanes.cu),
     // a larger one a thread per electron
-    int group = 0;
+    int group = 0, sms = 0;
+    bool resident = false;
     if (block_size <= 0) {
         block_size = 128;
-        int dev = 0, sms = 0;
+        int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
             return MCD_ECUDA;
         group = lanes_per_electron(*sim, *mat, sms);
+        resident = group == 0 && one_block_per_sm(*sim, *mat, sms);
         // a thread per electron: 128 threads, halved (down to 8) while the
         // grid would leave SMs idle, so that a small job spreads over the GPU;
         // FP64 further, down to 2 while the grid stays within one warp per
@@ -519,6 +615,7 @@ extern "C" int mcd_run(const mcd_sim* sim, const mcd_material* mat, const mcd_ta
     }
     const SimConst<float> c = make_consts<float>(*sim, *mat, tm, tg);
     if (group) return launch_lanes<float>(c, group, tally, eo, rg, rec, status, st);
+    if (resident) return launch_run(c, sms, tally, electrons ? *electrons : mcd_electron_out{}, rg, rec, status, st);
     return dispatch_plain<float>(c, block_size, tally, eo, rg, rec, status, st);
 }
 
@@ -619,41 +716,68 @@ extern "C" int mcd_batch_prepare(const mcd_sim* sims, int32_t nsims, const mcd_m
     return rc;
 }
 
+// The launch tuning of a batched run; MCD_OK or why it is refused.
+static int read_tune(const mcd_tune* tune, int* block, int* per_sm, int* refill) {
+    *block = 256;
+    *per_sm = 0;
+    *refill = 1;
+    if (tune) {
+        if (tune->block_size > 0) *block = tune->block_size;
+        if (tune->blocks_per_sm > 0) *per_sm = tune->blocks_per_sm;
+        if (tune->refill > 0) *refill = tune->refill;
+    }
+    if (*block % 32 != 0 || *block > 1024 || *refill < 1 || *refill > 32 || (tune && tune->reserved != 0))
+        return MCD_EINVAL;
+    return MCD_OK;
+}
+
+template <class K>
+static int set_smem(K kern, size_t smem) {
+    if (smem <= 48 * 1024) return MCD_OK;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess
+               ? MCD_OK
+               : MCD_ECUDA;
+}
+
+// The persistent launch and, where the list can hold an electron per lane and
+// the run-down kernel's block fits, that kernel after it.
+template <bool REC>
+static int launch_batched(void* workspace, int nsims, mcd_tally* tallies, const mcd_tune* tune,
+                          const mcd_event_ring& ring, uint32_t* status, bool lowreg, cudaStream_t st) {
+    int block, per_sm, refill;
+    if (read_tune(tune, &block, &per_sm, &refill) != MCD_OK) return MCD_EINVAL;
+    int flags = (tune && (tune->variant & 2)) ? kRunInline : 0;
+    if (lowreg && block > 576) return MCD_EINVAL;
+    int dev = 0, sms = 0, most = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return MCD_ECUDA;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return MCD_ECUDA;
+    if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return MCD_ECUDA;
+    const size_t smem = batch_smem(nsims), smem2 = batch_drain_off(nsims) + drain_smem(kDrainThreads);
+    auto kern = k_batched<REC>;
+    if constexpr (!REC) kern = lowreg ? k_batched_lr<false> : k_batched<false>;
+    if (set_smem(kern, smem) != MCD_OK) return MCD_ECUDA;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, block, smem) != cudaSuccess) return MCD_ECUDA;
+    if (fit < 1) return MCD_ETOOBIG;
+    if (per_sm <= 0 || per_sm > fit) per_sm = fit;
+    if ((long long)sms * per_sm * block <= kLiveSeats && smem2 + 1024 <= (size_t)most) flags |= kRunList;
+    if ((flags & kRunList) && set_smem(k_rundown<REC>, smem2) != MCD_OK) return MCD_ECUDA;
+    // reset the queue and the list (the first two words of the workspace)
+    if (cudaMemsetAsync(workspace, 0, 2 * sizeof(unsigned long long), st) != cudaSuccess) return MCD_ECUDA;
+    uint8_t* ws = static_cast<uint8_t*>(workspace);
+    kern<<<sms * per_sm, block, smem, st>>>(ws, tallies, refill, status, ring, flags);
+    if (cudaGetLastError() != cudaSuccess) return MCD_ECUDA;
+    if (flags & kRunList) k_rundown<REC><<<sms, kDrainThreads, smem2, st>>>(ws, tallies, status, ring, flags);
+    return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
+}
+
 extern "C" int mcd_run_batched(void* workspace, int32_t nsims, mcd_tally* tallies, const mcd_tune* tune,
                                uint32_t* status, void* stream) {
     if (!workspace || !tallies || !status) return MCD_EINVAL;
     if (nsims <= 0) return MCD_EINVAL;
     if (nsims > kBatchMaxSims) return MCD_ETOOBIG;
-    int block = 256, per_sm = 0, refill = 1;
-    if (tune) {
-        if (tune->block_size > 0) block = tune->block_size;
-        if (tune->blocks_per_sm > 0) per_sm = tune->blocks_per_sm;
-        if (tune->refill > 0) refill = tune->refill;
-    }
-    if (block % 32 != 0 || block > 1024 || refill < 1 || refill > 32 || (tune && tune->reserved != 0))
-        return MCD_EINVAL;
-    const bool lowreg = tune && (tune->variant & 1);
-    const int inline_sigma = (tune && (tune->variant & 2)) ? 1 : 0;
-    if (lowreg && block > 576) return MCD_EINVAL;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return MCD_ECUDA;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return MCD_ECUDA;
-    const size_t smem = batch_smem(nsims);
-    auto kern = lowreg ? k_batched_lr<false> : k_batched<false>;
-    if (smem > 48 * 1024) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return MCD_ECUDA;
-    }
-    int fit = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, block, smem) != cudaSuccess) return MCD_ECUDA;
-    if (fit < 1) return MCD_ETOOBIG;
-    if (per_sm <= 0 || per_sm > fit) per_sm = fit;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // reset the queue (the first word of the workspace)
-    if (cudaMemsetAsync(workspace, 0, sizeof(unsigned long long), st) != cudaSuccess) return MCD_ECUDA;
-    kern<<<sms * per_sm, block, smem, st>>>(static_cast<uint8_t*>(workspace), tallies, refill, status,
-                                            mcd_event_ring{}, inline_sigma);
-    return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
+    return launch_batched<false>(workspace, nsims, tallies, tune, mcd_event_ring{}, status,
+                                 tune && (tune->variant & 1), static_cast<cudaStream_t>(stream));
 }
 
 // Batched run that also appends every event to a device ring (the streaming
@@ -665,33 +789,8 @@ extern "C" int mcd_run_batched_ring(void* workspace, int32_t nsims, mcd_tally* t
     if (ring->fields & ~(MCD_EV_ALL | MCD_EV_PACKED_HEAD)) return MCD_EINVAL;
     if (nsims <= 0) return MCD_EINVAL;
     if (nsims > kBatchMaxSims) return MCD_ETOOBIG;
-    int block = 256, per_sm = 0, refill = 1;
-    if (tune) {
-        if (tune->block_size > 0) block = tune->block_size;
-        if (tune->blocks_per_sm > 0) per_sm = tune->blocks_per_sm;
-        if (tune->refill > 0) refill = tune->refill;
-    }
-    if (block % 32 != 0 || block > 1024 || refill < 1 || refill > 32 || (tune && tune->reserved != 0))
-        return MCD_EINVAL;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return MCD_ECUDA;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return MCD_ECUDA;
-    const size_t smem = batch_smem(nsims);
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(k_batched<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess)
-        return MCD_ECUDA;
-    int fit = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_batched<true>, block, smem) != cudaSuccess)
-        return MCD_ECUDA;
-    if (fit < 1) return MCD_ETOOBIG;
-    if (per_sm <= 0 || per_sm > fit) per_sm = fit;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (cudaMemsetAsync(workspace, 0, sizeof(unsigned long long), st) != cudaSuccess) return MCD_ECUDA;
-    const int inline_sigma = (tune && (tune->variant & 2)) ? 1 : 0;
-    k_batched<true><<<sms * per_sm, block, smem, st>>>(static_cast<uint8_t*>(workspace), tallies, refill, status,
-                                                          *ring, inline_sigma);
-    return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
+    return launch_batched<true>(workspace, nsims, tallies, tune, *ring, status, false,
+                                static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------
@@ -840,6 +939,6 @@ extern "C" int mcd_run_batched_noalloc(const mcd_sim* sims, int32_t nsims, const
     k_static_stage<<<(words + 255) / 256, 256, 0, st>>>(static_cast<uint4*>(scratch), blk, words);
     if (cudaGetLastError() != cudaSuccess) return MCD_ECUDA;
     kern<<<sms * per_sm, block, smem, st>>>(static_cast<uint8_t*>(scratch), tallies, refill, status,
-                                            mcd_event_ring{}, inline_sigma);
+                                            mcd_event_ring{}, inline_sigma ? kRunInline : 0);
     return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
 }

@@ -19,11 +19,12 @@ BUILD_DIR = os.path.join(ROOT, "_build")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
-SOURCES = ["mcd_host.cpp", "mcd_tables.cu", "mcd_transport.cu", "mcd_lanes.cu", "mcd_adjoint.cu", "mcd_detector.cu"]
+SOURCES = ["mcd_host.cpp", "mcd_tables.cu", "mcd_transport.cu", "mcd_lanes.cu", "mcd_run.cu", "mcd_adjoint.cu", "mcd_detector.cu"]
 EXTRA = {
     # FP32 transport: approximate division/sqrt and flush-to-zero; FP64
     # transport is unaffected by these flags.
     "mcd_transport.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false", "-Xptxas", "-v"],
+    "mcd_run.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
     "mcd_lanes.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false"],
     "mcd_adjoint.cu": ["-ftz=true", "-prec-div=false", "-prec-sqrt=false", "--extended-lambda"],
 }
