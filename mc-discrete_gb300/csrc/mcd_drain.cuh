@@ -208,6 +208,14 @@ __device__ __forceinline__ uint32_t group_run(const Sims& s, int sim, Lane<float
         }
         next = buf[g.h0 + ((k + 1) & (G - 1))];
         EventOut<float> ev;
+        RingTicket tk{};
+        uint32_t el = 0;
+        if (REC) {
+            el = (uint32_t)(elec_index(c, rng) - c.first);
+            const bool rec = g.t == 0 && have && L.step < w.w;
+            tk = ring_reserve(ring, rec && ring_takes(ring, el));
+            if (rec && !ring_takes(ring, el)) st |= MCD_FLAG_RING_INDEX;
+        }
         int ch = kGroupNone;
         if (Sims::MODE != MCD_MODE_CONT)
             ch = group_event<float, REC, G>(L, sig, c, cur, have && !cont, w.w, g, zmax, use_tab, &ev);
@@ -219,8 +227,7 @@ __device__ __forceinline__ uint32_t group_run(const Sims& s, int sim, Lane<float
                 ch = cont_event_r<float, REC>(L, c, make_uint4(0u, 0u, cur.rz, cur.rw), &ev, &cur);
             }
         }
-        if (REC && g.t == 0 && ch != kGroupNone)
-            st |= ring_append(ring, (uint32_t)(elec_index(c, rng) - c.first), L.step, ev);
+        if (REC) ring_write(ring, ring_slot(ring, tk), el, L.step, ev);
         if (ch != kGroupPlain && have) {
             if (CHAN && g.t == 0 && ch > MCD_CH_RUTH) atomicAdd(&s.t(sim).channel[ch], 1ull);
             if (L.outcome != MCD_OUT_NONE) {
@@ -297,10 +304,18 @@ __device__ __forceinline__ uint32_t drain_run(const Sims& run, unsigned count, T
     auto event = [&]() {
         const SimConst<float>& c = run.c(sim);
         EventOut<float> ev;
+        RingTicket tk{};
+        uint32_t el = 0;
+        if (REC) {
+            el = (uint32_t)(elec_index(c, rng) - c.first);
+            const bool rec = L.step < c.max_scatt;
+            tk = ring_reserve(ring, rec && ring_takes(ring, el));
+            if (rec && !ring_takes(ring, el)) st |= MCD_FLAG_RING_INDEX;
+        }
         int ch;
         if (run_cont<Sims>(c)) ch = cont_event<float, REC>(L, c, rng, &ev);
         else ch = ds_event<float, REC>(L, c, rng, &ev, !inline_sigma && c.sig != nullptr);
-        if (REC && ch >= 0) st |= ring_append(ring, (uint32_t)(elec_index(c, rng) - c.first), L.step, ev);
+        if (REC) ring_write(ring, ring_slot(ring, tk), el, L.step, ev);
         if (CHAN && ch > MCD_CH_RUTH) atomicAdd(&run.t(sim).channel[ch], 1ull);
         if (L.outcome != MCD_OUT_NONE) {
             st |= run_finish(run, sim, L, rng);

@@ -283,12 +283,20 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
         if (have) {
             const SimConst<float>& c = s_c[sim];
             EventOut<float> ev;
+            RingTicket tk{};
+            uint32_t el = 0;
+            if (REC) {
+                el = (uint32_t)(elec_index(c, rng) - c.first);
+                const bool rec = L.step < c.max_scatt;
+                tk = ring_reserve(ring, rec && ring_takes(ring, el));
+                if (rec && !ring_takes(ring, el)) st |= MCD_FLAG_RING_INDEX;
+            }
             int ch;
             if (!(c.bits & kBitCont))
                 ch = ds_event<float, REC>(L, c, rng, &ev, !inline_sigma && c.sig != nullptr);
             else
                 ch = cont_event<float, REC>(L, c, rng, &ev);
-            if (REC && ch >= 0) st |= ring_append(ring, (uint32_t)(elec_index(c, rng) - c.first), L.step, ev);
+            if (REC) ring_write(ring, ring_slot(ring, tk), el, L.step, ev);
             if (CHAN && ch > MCD_CH_RUTH) atomicAdd(&s_t[sim].channel[ch], 1ull);
             if (L.outcome != MCD_OUT_NONE) {
                 const mcd_electron_out& r = rows[sim];
