@@ -150,18 +150,21 @@ struct ManySims {
     mcd_tally* tallies_;
     const mcd_electron_out* rows_;
     __device__ __forceinline__ const SimConst<float>& c(int sim) const { return c_[sim]; }
+    __device__ __forceinline__ const SimConst<float>& full(int sim) const { return c_[sim]; }
     __device__ __forceinline__ BlockTally& t(int sim) const { return t_[sim]; }
     __device__ __forceinline__ mcd_tally* tally(int sim) const { return tallies_ + sim; }
     __device__ __forceinline__ const mcd_electron_out& rows(int sim) const { return rows_[sim]; }
 };
-template <int M>
+template <int M, class C>
 struct OneSim {
     static constexpr int MODE = M;
-    const SimConst<float>& c_;
+    const SimConst<float>& full_;
+    const C& c_;   // what its events read: the same, or a HotConst
     BlockTally& t_;
     mcd_tally* tally_;
     const mcd_electron_out& rows_;
-    __device__ __forceinline__ const SimConst<float>& c(int) const { return c_; }
+    __device__ __forceinline__ const C& c(int) const { return c_; }
+    __device__ __forceinline__ const SimConst<float>& full(int) const { return full_; }
     __device__ __forceinline__ BlockTally& t(int) const { return t_; }
     __device__ __forceinline__ mcd_tally* tally(int) const { return tally_; }
     __device__ __forceinline__ const mcd_electron_out& rows(int) const { return rows_; }
@@ -169,7 +172,7 @@ struct OneSim {
 
 template <class Sims>
 __device__ __forceinline__ uint32_t run_finish(const Sims& s, int sim, const Lane<float>& L, const ElecRng& rng) {
-    const SimConst<float>& c = s.c(sim);
+    const SimConst<float>& c = s.full(sim);
     const mcd_electron_out& r = s.rows(sim);
     const ElOut eo{r.outcome, r.flags, r.final_E, r.dir, r.last_pos, r.max_z, r.n_events};
     return finish_electron(c, L, elec_index(c, rng) - c.first, s.t(sim), s.tally(sim), eo);
@@ -187,7 +190,7 @@ __device__ __forceinline__ uint32_t group_run(const Sims& s, int sim, Lane<float
                                               bool inline_sigma) {
     const int lane = threadIdx.x & 31;
     const GroupLanes<G> g(lane);
-    const SimConst<float>& c = s.c(sim);
+    const auto& c = s.c(sim);
     const uint4 w = event_words(c);
     const bool cont = run_cont<Sims>(c);
     const bool use_tab = !inline_sigma && c.sig != nullptr;
@@ -211,7 +214,7 @@ __device__ __forceinline__ uint32_t group_run(const Sims& s, int sim, Lane<float
         RingTicket tk{};
         uint32_t el = 0;
         if (REC) {
-            el = (uint32_t)(elec_index(c, rng) - c.first);
+            el = (uint32_t)(elec_index(s.full(sim), rng) - s.full(sim).first);
             const bool rec = g.t == 0 && have && L.step < w.w;
             tk = ring_reserve(ring, rec && ring_takes(ring, el));
             if (rec && !ring_takes(ring, el)) st |= MCD_FLAG_RING_INDEX;
@@ -302,13 +305,13 @@ __device__ __forceinline__ uint32_t drain_run(const Sims& run, unsigned count, T
     bool have = (threadIdx.x >> 5) < wide && first < count;
     if (have) take(first, L, rng, sim);
     auto event = [&]() {
-        const SimConst<float>& c = run.c(sim);
+        const auto& c = run.c(sim);
         EventOut<float> ev;
         RingTicket tk{};
         uint32_t el = 0;
         if (REC) {
-            el = (uint32_t)(elec_index(c, rng) - c.first);
-            const bool rec = L.step < c.max_scatt;
+            el = (uint32_t)(elec_index(run.full(sim), rng) - run.full(sim).first);
+            const bool rec = L.step < event_words(c).w;
             tk = ring_reserve(ring, rec && ring_takes(ring, el));
             if (rec && !ring_takes(ring, el)) st |= MCD_FLAG_RING_INDEX;
         }

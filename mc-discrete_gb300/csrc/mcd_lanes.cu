@@ -25,27 +25,36 @@
 
 namespace mcd {
 
+// Blocks per SM that the registers must leave room for: what the automatic
+// rule gives an SM at most (in FP64 the narrow groups' alone; spilling more
+// there costs as much as it gains).
+template <class T>
+constexpr int lanes_blocks(int group) {
+    return sizeof(T) == 4 ? (group == 8 ? 20 : 16) : (group == 8 ? 16 : 1);
+}
+
 template <class T, int MODE, bool REC, int G>
-__global__ void __launch_bounds__(32) k_lanes(const SimConst<T> cp, mcd_tally* tally, const ElOut eo,
+__global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst<T> cp, mcd_tally* tally, const ElOut eo,
                                               const mcd_event_ring ring, uint32_t* status) {
     __shared__ BlockTally bt;
-    __shared__ SimConst<T> c;
+    __shared__ SimConst<T> full;
     __shared__ EventPre<T> pre[2][32];
-    if (threadIdx.x == 0) c = cp;
+    if (threadIdx.x == 0) full = cp;
     bt_zero(&bt, 1);
     __syncwarp();
+    const HotConst<T> c(full);
     const int lane = threadIdx.x;
     const GroupLanes<G> g(lane);
     const uint64_t i = (uint64_t)blockIdx.x * (32 / G) + (uint64_t)(lane / G);
-    bool active = i < (uint64_t)c.num_el;
-    const ElecRng rng = elec_rng(c, c.first + i);
+    bool active = i < (uint64_t)full.num_el;
+    const ElecRng rng = elec_rng(full, full.first + i);
     const uint4 w = event_words(c);   // sim id and Philox key words, event limit
-    const bool chan = (c.tally_flags & MCD_TALLY_CHANNELS) != 0;
+    const bool chan = (full.tally_flags & MCD_TALLY_CHANNELS) != 0;
     const T zmax = group_zmax<T>(c);
     const bool use_tab = c.sig != nullptr;
     const T ang = MODE == MCD_MODE_DS ? c.a0 : (T)1;
     Lane<T> L;
-    lane_init(L, c);
+    lane_init(L, full);
     GroupSig<T, G> sig;
     if (MODE == MCD_MODE_DS) group_sig<T, G>(c, L.E, use_tab, g.t, g.h0, g.gmask, sig);
     // every electron of the warp that still runs is at the same event
@@ -75,7 +84,7 @@ __global__ void __launch_bounds__(32) k_lanes(const SimConst<T> cp, mcd_tally* t
         if (ch != kGroupPlain && active) {
             if (g.t == 0 && chan && ch > MCD_CH_RUTH) atomicAdd(&bt.channel[ch], 1ull);
             if (L.outcome != MCD_OUT_NONE) {
-                if (g.t == 0) st |= finish_electron(c, L, i, bt, tally, eo);
+                if (g.t == 0) st |= finish_electron(full, L, i, bt, tally, eo);
                 active = false;
             }
         }

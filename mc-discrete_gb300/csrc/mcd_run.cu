@@ -9,6 +9,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "mcd_drain.cuh"
 #include "mcd_run.h"
 
@@ -27,7 +29,13 @@ __global__ void __launch_bounds__(THREADS) k_run(const SimConst<float> cp, mcd_t
     }
     bt_zero(&bt, 1);
     __syncthreads();
-    const OneSim<MODE> run{c, bt, tally, rows};
+    // 1024 threads leave no registers for the constants
+    using C = typename std::conditional<THREADS == 512, HotConst<float>, SimConst<float>>::type;
+    const HotConst<float> hot(c);
+    const C* pc;
+    if constexpr (THREADS == 512) pc = &hot;
+    else pc = &c;
+    const OneSim<MODE, C> run{c, *pc, bt, tally, rows};
     const unsigned count = (unsigned)(((unsigned long long)c.num_el - blockIdx.x + gridDim.x - 1) / gridDim.x);
     auto take = [&](unsigned k, Lane<float>& L, ElecRng& rng, int& sim) {
         rng = elec_rng(c, c.first + blockIdx.x + (uint64_t)k * gridDim.x);

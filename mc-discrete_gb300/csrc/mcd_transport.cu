@@ -515,13 +515,16 @@ static int dispatch_plain(const SimConst<T>& c, int block, mcd_tally* tally, con
 // electron.  More lanes make an electron's chain shorter, but a warp issues
 // for fewer electrons, so the width falls as the run fills the GPU; the lines
 // (in electrons per SM) lie where the two sides measured equal on 152 SMs,
-// kernel times in ms, 0 = a thread per electron:
-//   FP32 DS (Si, table)  1000: 0.30 with 32, 0.58 with 0;  3500: 0.45 / 0.46
-//                        with 32 / 16;  5000: 0.53 / 0.55 with 16 / 8;
-//                        10000: 0.73 / 0.77 with 8 / 0;  14000: 1.05 / 0.77
-//   (Au: 10000 1.93 / 3.01 with 8 / 0, 20000 3.14 / 2.97; Cu without a table:
-//   10000 1.44 / 1.97, 14000 2.03 / 1.97)
-//   FP32 continuous      1000: 0.23 / 0.27 with 32 / 0;  2500: 0.31 / 0.28
+// kernel times in ms, 0 = a thread per electron (in FP32 DS as mcd_run.cu runs
+// it):
+//   FP32 DS (Si, table)  2500: 0.35 / 0.39 with 32 / 16;  3500: 0.49 / 0.43;
+//                        4500: 0.48 / 0.49 with 16 / 8;  7500: 0.55 / 0.56
+//                        with 8 / 0;  10000: 0.67 / 0.59
+//   (Au: 3500 1.07 / 1.26 with 32 / 16, 4500 1.35 / 1.34 with 16 / 8, 7500
+//   1.53 / 1.63 with 8 / 0, 10000 1.83 / 1.72; Cu without a table: 3500 0.88 /
+//   0.85, 4500 0.95 / 1.08, 7500 1.21 / 1.23, 10000 1.36 / 1.32)
+//   FP32 continuous      1500: 0.21 / 0.23 with 32 / 8;  2500: 0.28 / 0.24;
+//                        4500: 0.25 / 0.27 with 8 / 0;  6500: 0.28 / 0.28
 //   FP64 DS (Si, table)  700: 2.27 / 2.38 with 32 / 16;  1500: 2.65 / 2.66 with
 //                        16 / 8;  3500: 3.48 / 4.35 with 8 / 0;  5000: 4.96 / 4.76
 //   without a table      Si 5000: 13.3 / 14.7 with 8 / 0, 7500 19.7 / 15.3;
@@ -532,8 +535,8 @@ static int dispatch_plain(const SimConst<T>& c, int block, mcd_tally* tally, con
 static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) {
     const int64_t e = s.num_el / sms;   // electrons per SM
     if (s.precision == MCD_FP32) {
-        if (s.mode != MCD_MODE_DS) return e < 10 ? 32 : 0;
-        return e < 23 ? 32 : e < 33 ? 16 : e < 70 ? 8 : 0;
+        if (s.mode != MCD_MODE_DS) return e < 12 ? 32 : e < 34 ? 8 : 0;
+        return e < 20 ? 32 : e < 33 ? 16 : e < 58 ? 8 : 0;
     }
     if (s.mode != MCD_MODE_DS) return e < 3 ? 32 : e < 10 ? 8 : 0;
     const int most = s.sigma_table ? 28 : 12 * (m.n_shells > 3 ? m.n_shells : 3);
@@ -545,21 +548,20 @@ static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) 
 // independent threads?  The first keeps warps full where trajectory lengths
 // differ; its barriers and its own loop cost a few percent where they do not.
 // Kernel times in ms, this against independent threads:
-//   FP32 DS    from 70 electrons per SM, where the lanes of mcd_lanes.cu end
-//              (20000 electrons: Cu 1.85 / 2.00, Au 2.37 / 2.98, Si 0.74 / 0.77;
-//              40000: Cu 2.10 / 2.21, Au 2.99 / 3.36, Si 0.87 / 0.83; 1e6: Cu
-//              12.6 / 21.5, Au 14.0 / 33.4, Si 6.1 / 8.0)
+//   FP32 DS    always (10000 electrons: Cu 1.32 / 1.96, Au 1.72 / 2.74, Si 0.59
+//              / 0.75; 80000: Cu 2.39 / 2.66, Au 3.39 / 4.01, Si 0.98 / 0.98;
+//              1e6: Cu 12.6 / 21.5, Au 14.0 / 33.4, Si 6.1 / 8.0)
 //   FP32 continuous, whose lengths differ by backscattering alone: 1e6
 //              electrons Cu 70 deg 2.64 / 4.26, Al 70 deg 1.77 / 2.27, Au 0 deg
-//              7.5 / 10.8, Cu 0 deg 3.97 / 4.30, but Al 0 deg 2.39 / 2.28; from
-//              one wave of lanes on (150000: Cu 70 deg 0.55 / 0.77; 80000:
-//              0.43 / 0.49; 40000: 0.38 / 0.36)
+//              7.5 / 10.8, Cu 0 deg 3.97 / 4.30, but Al 0 deg 2.39 / 2.28;
+//              (Cu 70 deg 100000: 0.48 / 0.58, 40000: 0.33 / 0.36, 10000: 0.28
+//              / 0.28)
 static bool one_block_per_sm(const mcd_sim& s, const mcd_material& m, int sms) {
     const int64_t e = s.num_el / sms;   // electrons per SM
     if (s.precision != MCD_FP32 || e > INT32_MAX / 2) return false;
-    if (s.mode == MCD_MODE_DS) return e >= 70;
+    if (s.mode == MCD_MODE_DS) return true;
     if (s.E0 < 10.0 * s.Emin) return false;   // short trajectories: the start and the end weigh more
-    if (s.s_tilt >= 60.0 || m.Z >= 40) return e >= 450;
+    if (s.s_tilt >= 60.0 || m.Z >= 40) return e >= 230;
     return m.Z >= 25 && e >= 4000;
 }
 

@@ -22,7 +22,7 @@ RUNS = {
     "cont_ex": dict(input_par("Al", 5000.0, 1000.0, 0.0, mode="cont", bethe="explicit"), maxScatt=150),
 }
 SMS = 152
-# electrons per SM: below 3, 5, 10, 23, 33 and 70 the group width changes
+# electrons per SM: below 3, 5, 10, 12, 20, 33 and 58 the group width changes
 SIZES = [1, 2, 3, 31, 2 * SMS + 1, 4 * SMS, 9 * SMS + 5, 11 * SMS, 25 * SMS + 3, 40 * SMS + 7]
 
 
