@@ -69,8 +69,10 @@ class ExitEnergyModel:
         self.queue = torch.zeros(1, dtype=torch.int64, device=self.device)   # the forward pass's work queue
         self.buf = AdjointBuf(self.ckpt.data_ptr(), self.kstar.data_ptr(), self.E_exit.data_ptr(), self.max_ckpt, 0,
                               self.queue.data_ptr())
-        self.hout = torch.zeros(self.nbins + 2, dtype=torch.float64, device=self.device)
-        self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
+        # the bins and, in the last word, the status: cleared and read as one
+        self._out = torch.zeros(self.nbins + 3, dtype=torch.float64, device=self.device)
+        self.hout = self._out[:self.nbins + 2]
+        self.status = self._out[self.nbins + 2:].view(torch.int32)[:1]
         self.grad = torch.zeros(2, dtype=torch.float64, device=self.device)
         self.grad_in = torch.zeros(self.nbins + 1, dtype=torch.float64, device=self.device)
 
@@ -83,8 +85,7 @@ class ExitEnergyModel:
 
     def launch_forward(self, J_scale=1.0, n_scale=1.0):
         """Enqueue the forward pass (no host synchronisation)."""
-        self.hout.zero_()
-        self.status.zero_()
+        self._out.zero_()
         s = self.sim(J_scale, n_scale)
         code = _lib.lib().mcd_adjoint_forward(C.byref(s), C.byref(self.mat), C.byref(self.hist), C.byref(self.buf),
                                               self.hout.data_ptr(), None, self.status.data_ptr(), self._stream())
@@ -95,12 +96,12 @@ class ExitEnergyModel:
         """Soft bins h_b (normalised by N), sum of exit energies, number of 'bks'."""
         while True:
             self.launch_forward(J_scale, n_scale)
-            st = int(self.status.item())
+            h = self._out.cpu().numpy()
+            st = int(h[self.nbins + 2:].view(np.int32)[0])
             if not (st & _lib.FLAG_CKPT):   # an exiting electron outran the checkpoint slots
                 break
             self.max_ckpt *= 2
             self._alloc()
-        h = self.hout.cpu().numpy()
         return h[:self.nbins] / self.n, float(h[self.nbins]), float(h[self.nbins + 1])
 
     def launch_backward(self, grad_h, grad_sum):

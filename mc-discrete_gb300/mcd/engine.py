@@ -119,36 +119,71 @@ def use_sigma_table(sim, mat, device="cuda"):
     return t
 
 
-def tally_to_dict(t):
-    out = {k: int(t.outcome[i]) for i, k in enumerate(_lib.OUTCOME_NAMES)}
-    for k in ("events", "double_rows", "nan_events", "clamped", "long_path", "table_range"):
-        out[k] = int(getattr(t, k))
-    out["channel"] = np.array(t.channel[:], dtype=np.int64)
-    out["sum_E_bks"] = float(t.sum_E_bks)
-    out["sum_E2_bks"] = float(t.sum_E2_bks)
-    out["sum_steps2"] = float(t.sum_steps2)
-    out["hist_E"] = np.array(t.hist_E[:], dtype=np.int64)
-    out["hist_T"] = np.array(t.hist_T[:], dtype=np.int64)
-    return out
+_TALLY_WORDS = [(f[0], getattr(_lib.Tally, f[0]).offset // 8, getattr(_lib.Tally, f[0]).size // 8)
+                for f in _lib.Tally._fields_]
 
 
 def tally_from_bytes(buf):
-    t = _lib.Tally.from_buffer_copy(bytes(buf))
-    return tally_to_dict(t)
+    """An mcd_tally's bytes as a dict."""
+    w = np.frombuffer(bytes(buf), dtype=np.int64)
+    f = {k: w[a:a + n] for k, a, n in _TALLY_WORDS}
+    out = {k: int(f["outcome"][i]) for i, k in enumerate(_lib.OUTCOME_NAMES)}
+    for k in ("events", "double_rows", "nan_events", "clamped", "long_path", "table_range"):
+        out[k] = int(f[k][0])
+    out["channel"] = f["channel"].copy()
+    for k in ("sum_E_bks", "sum_E2_bks", "sum_steps2"):
+        out[k] = float(f[k].view(np.float64)[0])
+    out["hist_E"] = f["hist_E"].copy()
+    out["hist_T"] = f["hist_T"].copy()
+    return out
 
 
-def _device_rows(n, fdt, device):
-    """Per-electron row arrays on the device (the mcd_electron_out layout)."""
+def tally_to_dict(t):
+    return tally_from_bytes(bytes(t))
+
+
+_ALIGN = 512   # bytes; as the allocator aligns tensors of their own
+
+
+class _Store:
+    """Zeroed device arrays of one run in one allocation, so that they are
+    cleared by one fill and read back by one copy: a small run's fills and
+    copies, one per array, took about as long as its transport.
+
+    add(dtype, n) reserves an array and returns its number, make(device)
+    allocates, self[k] is array k on the device, and host() reads everything
+    back once and returns k -> array k in host memory."""
+
+    def __init__(self):
+        self.spans, self.size = [], 0
+
+    def add(self, dtype, n):
+        nbytes = n * dtype.itemsize
+        self.spans.append((dtype, self.size, nbytes))
+        self.size += -(-nbytes // _ALIGN) * _ALIGN
+        return len(self.spans) - 1
+
+    def make(self, device):
+        torch = _torch()
+        self.bytes = torch.zeros(max(self.size, 1), dtype=torch.uint8, device=device)
+        self.arrays = [self.bytes[a:a + n].view(dt) for dt, a, n in self.spans]
+
+    def __getitem__(self, k):
+        return self.arrays[k]
+
+    def host(self):
+        b = self.bytes.cpu()
+        return lambda k: b[self.spans[k][1]:self.spans[k][1] + self.spans[k][2]].view(self.spans[k][0]).numpy()
+
+
+_ROWS = ("outcome", "flags", "final_E", "dir", "last_pos", "max_z", "n_events")
+
+
+def _add_rows(store, n, fdt):
+    """Reserves the per-electron row arrays (the mcd_electron_out layout)."""
     torch = _torch()
-    return dict(
-        outcome=torch.zeros(n, dtype=torch.uint8, device=device),
-        flags=torch.zeros(n, dtype=torch.uint8, device=device),
-        final_E=torch.zeros(n, dtype=fdt, device=device),
-        dir=torch.zeros(3 * n, dtype=fdt, device=device),
-        last_pos=torch.zeros(3 * n, dtype=fdt, device=device),
-        max_z=torch.zeros(n, dtype=fdt, device=device),
-        n_events=torch.zeros(n, dtype=torch.int32, device=device),
-    )
+    kinds = ((torch.uint8, n), (torch.uint8, n), (fdt, n), (fdt, 3 * n), (fdt, 3 * n), (fdt, n), (torch.int32, n))
+    return {k: store.add(dt, m) for k, (dt, m) in zip(_ROWS, kinds)}
 
 
 def _rows_struct(e):
@@ -157,12 +192,16 @@ def _rows_struct(e):
                             e["n_events"].data_ptr())
 
 
-def _host_rows(el, n):
-    """Per-electron rows copied to the host (dir and last_pos as (n, 3))."""
-    e = {k: v.cpu().numpy() for k, v in el.items()}
-    return dict(outcome=e["outcome"], flags=e["flags"], final_E=e["final_E"],
-                dir=e["dir"].reshape(3, n).T.copy(), last_pos=e["last_pos"].reshape(3, n).T.copy(),
-                max_z=e["max_z"], n_events=e["n_events"])
+_DEVICE_TRANSPOSE = 8192   # electrons from which the device turns the planes (100000: 15 us against 320 in NumPy)
+
+
+def _host_rows(el, n, host):
+    """Per-electron rows on the host (dir and last_pos as (n, 3)); el: the
+    device arrays, host(name): their copies on the host."""
+    e = {k: host(k) for k in _ROWS if n < _DEVICE_TRANSPOSE or k not in ("dir", "last_pos")}
+    for k in ("dir", "last_pos"):
+        e[k] = e[k].reshape(3, n).T.copy() if k in e else el[k].view(3, n).t().contiguous().cpu().numpy()
+    return {k: e[k] for k in ("outcome", "flags", "final_E", "dir", "last_pos", "max_z", "n_events")}
 
 
 class RunBuffers:
@@ -173,23 +212,24 @@ class RunBuffers:
         self.device = torch.device(device)
         self.num_el = int(num_el)
         self.precision = precision
-        tsz = C.sizeof(_lib.Tally)
-        self.tally = torch.zeros(tsz, dtype=torch.uint8, device=self.device)
-        self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
         fdt = torch.float32 if precision == _lib.FP32 else torch.float64
-        self.el = _device_rows(self.num_el, fdt, self.device) if electrons else None
+        st = self._store = _Store()
+        tally, status, cursor = st.add(torch.uint8, C.sizeof(_lib.Tally)), st.add(torch.int32, 1), st.add(torch.int64, 1)
+        self._head = st.size      # what a launch adds to: cleared before each
+        self._rows = _add_rows(st, self.num_el, fdt) if electrons else None
+        st.make(self.device)
+        self.tally, self.status = st[tally], st[status]
+        self._read = (tally, status, cursor)
+        self.el = {k: st[i] for k, i in self._rows.items()} if electrons else None
         self.ring = None
         self.ring_fields = int(ring_fields)
         if ring_capacity:
             self.ring = torch.zeros((int(ring_capacity), event_bytes(self.ring_fields)), dtype=torch.uint8,
                                     device=self.device)
-            self.cursor = torch.zeros(1, dtype=torch.int64, device=self.device)
+            self.cursor = st[cursor]
 
     def zero(self):
-        self.tally.zero_()
-        self.status.zero_()
-        if self.ring is not None:
-            self.cursor.zero_()
+        self._store.bytes[:self._head].zero_()
 
     def electron_struct(self):
         return _rows_struct(self.el) if self.el is not None else None
@@ -284,12 +324,14 @@ def launch(sim, mat, tables, bufs, block_size=0, stream=None):
 
 def collect(bufs):
     """Copy the results of the last launch back to the host (synchronises)."""
-    tally = tally_from_bytes(bufs.tally.cpu().numpy())
-    status = int(bufs.status.item())
-    electrons = _host_rows(bufs.el, bufs.num_el) if bufs.el is not None else None
+    host = bufs._store.host()
+    k_tally, k_status, k_cursor = bufs._read
+    tally = tally_from_bytes(host(k_tally))
+    status = int(host(k_status)[0])
+    electrons = _host_rows(bufs.el, bufs.num_el, lambda k: host(bufs._rows[k])) if bufs.el is not None else None
     events, total = None, 0
     if bufs.ring is not None:
-        total = int(bufs.cursor.item())
+        total = int(host(k_cursor)[0])
         k = min(total, bufs.ring.shape[0])
         events = bufs.ring[:k].cpu().numpy().view(event_dtype(bufs.ring_fields)).reshape(-1)
         if total > bufs.ring.shape[0]:
@@ -316,8 +358,7 @@ def run(input_par, num_el=None, seed=0, first_electron=0, precision="fp32", elec
         tables = ds_tables(mat, p["E0"], p["Emin"], p["Wc"], p["tol_E"], p["tol_W"], device)
     if tabulated:
         use_sigma_table(sim, mat, device)
-    bufs = RunBuffers(n, prec, electrons, ring_capacity, device, ring_fields)
-    bufs.zero()
+    bufs = RunBuffers(n, prec, electrons, ring_capacity, device, ring_fields)   # zeroed
     launch(sim, mat, tables if sim.mode == _lib.MODE_DS else None, bufs, block_size)
     return collect(bufs)
 
@@ -366,7 +407,13 @@ class Batch:
         self.tables = tabs
         self.el, self._el_structs = None, []
         if electrons:
-            self.el = [_device_rows(int(p["num_el"]), torch.float32, self.device) for p in self.inputs]
+            self.el, self._el_stores = [], []
+            for p in self.inputs:
+                st = _Store()
+                rows = _add_rows(st, int(p["num_el"]), torch.float32)
+                st.make(self.device)
+                self._el_stores.append((st, rows))
+                self.el.append({k: st[i] for k, i in rows.items()})
             self._el_structs = [_rows_struct(e) for e in self.el]   # read when the batch is packed
             for s_, eo in zip(self.structs, self._el_structs):
                 s_.electrons = C.addressof(eo)
@@ -445,4 +492,6 @@ class Batch:
         """Simulation k's per-electron rows on the host (electrons=True)."""
         if self.el is None:
             raise RuntimeError("the batch keeps no per-electron rows (electrons=False)")
-        return _host_rows(self.el[k], int(self.inputs[k]["num_el"]))
+        st, rows = self._el_stores[k]
+        host = st.host()
+        return _host_rows(self.el[k], int(self.inputs[k]["num_el"]), lambda name: host(rows[name]))

@@ -70,3 +70,23 @@ def test_batch_events_keep_their_order():
     r = engine.run(dict(RUNS["au"]), num_el=3000, seed=3, ring_capacity=3000 * 400, ring_fields=fields, block_size=64)
     assert total == r.events_total
     assert ev.tobytes() == r.events.tobytes()
+
+
+@pytest.mark.parametrize("n", [1, 8191, 8192, 20001])
+@pytest.mark.parametrize("precision", [_lib.FP32, _lib.FP64])
+def test_rows_read_back_are_the_device_arrays(n, precision):
+    p = dict(RUNS["cont"], maxScatt=20)
+    bufs = engine.RunBuffers(n, precision, ring_capacity=30 * n)
+    bufs.zero()
+    engine.launch(engine.make_sim(p, n, 1, precision=precision), _lib.material(p["material"]), None, bufs)
+    r = engine.collect(bufs)
+    el = {k: v.cpu().numpy() for k, v in bufs.el.items()}
+    for k in ("outcome", "flags", "final_E", "max_z", "n_events"):
+        assert np.array_equal(r.electrons[k], el[k]), k
+    for k in ("dir", "last_pos"):
+        assert r.electrons[k].shape == (n, 3) and r.electrons[k].flags.c_contiguous
+        assert np.array_equal(r.electrons[k], el[k].reshape(3, n).T), k
+    assert r.tally["events"] == int(el["n_events"].sum()) == r.events_total == int(bufs.cursor.item())
+    t = _lib.Tally.from_buffer_copy(bufs.tally.cpu().numpy().tobytes())
+    assert list(t.channel) == r.tally["channel"].tolist() and t.sum_E_bks == r.tally["sum_E_bks"]
+    assert list(t.hist_E) == r.tally["hist_E"].tolist() and list(t.hist_T) == r.tally["hist_T"].tolist()
