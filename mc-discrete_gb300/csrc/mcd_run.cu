@@ -4,17 +4,22 @@
 // Block b runs every gridDim.x-th electron: its lanes take the next of its
 // share as they fall idle, and when the share is handed out the block runs down
 // with compaction (mcd_drain.cuh).  No queue in global memory is needed, since
-// the shares of the SMs are statistically alike.  512 threads where they hold
-// the share (more registers, less to meet at a barrier), 1024 beyond.
+// the shares of the SMs are statistically alike.
 #include <cuda_runtime.h>
 #include <stdint.h>
-
-#include <type_traits>
 
 #include "mcd_drain.cuh"
 #include "mcd_run.h"
 
 namespace mcd {
+
+// Threads of a block: 512 where they hold its share of the electrons, else as
+// many as leave 72 registers each, enough for the constants (HotConst).
+// Against 1024 threads at 64 registers, with the constants in shared memory:
+// 1e6 electrons Si 5.65 / 6.04 ms, Au 12.9 / 13.5, Cu without a table 12.6 /
+// 12.5, continuous Cu 70 deg 2.50 / 2.65; 1e5: Si 0.94 / 1.06, Au 3.28 / 3.54,
+// Cu 2.39 / 2.54; 768 threads lose 2 to 8% of the large runs.
+constexpr int kThreadsMost = 896;
 
 template <int MODE, bool REC, int THREADS>
 __global__ void __launch_bounds__(THREADS) k_run(const SimConst<float> cp, mcd_tally* tally, const mcd_electron_out eo,
@@ -29,13 +34,8 @@ __global__ void __launch_bounds__(THREADS) k_run(const SimConst<float> cp, mcd_t
     }
     bt_zero(&bt, 1);
     __syncthreads();
-    // 1024 threads leave no registers for the constants
-    using C = typename std::conditional<THREADS == 512, HotConst<float>, SimConst<float>>::type;
     const HotConst<float> hot(c);
-    const C* pc;
-    if constexpr (THREADS == 512) pc = &hot;
-    else pc = &c;
-    const OneSim<MODE, C> run{c, *pc, bt, tally, rows};
+    const OneSim<MODE, HotConst<float>> run{c, hot, bt, tally, rows};
     const unsigned count = (unsigned)(((unsigned long long)c.num_el - blockIdx.x + gridDim.x - 1) / gridDim.x);
     auto take = [&](unsigned k, Lane<float>& L, ElecRng& rng, int& sim) {
         rng = elec_rng(c, c.first + blockIdx.x + (uint64_t)k * gridDim.x);
@@ -58,7 +58,7 @@ static int launch_threads(const SimConst<float>& c, int sms, mcd_tally* tally, c
     if (c.num_el <= (int64_t)512 * sms)
         k_run<MODE, REC, 512><<<grid, 512, drain_smem(512), st>>>(c, tally, rows, ring, status);
     else
-        k_run<MODE, REC, 1024><<<grid, 1024, drain_smem(1024), st>>>(c, tally, rows, ring, status);
+        k_run<MODE, REC, kThreadsMost><<<grid, kThreadsMost, drain_smem(kThreadsMost), st>>>(c, tally, rows, ring, status);
     return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
 }
 

@@ -549,10 +549,10 @@ static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) 
 // differ; its barriers and its own loop cost a few percent where they do not.
 // Kernel times in ms, this against independent threads:
 //   FP32 DS    always (10000 electrons: Cu 1.32 / 1.96, Au 1.72 / 2.74, Si 0.59
-//              / 0.75; 80000: Cu 2.39 / 2.66, Au 3.39 / 4.01, Si 0.98 / 0.98;
-//              1e6: Cu 12.6 / 21.5, Au 14.0 / 33.4, Si 6.1 / 8.0)
+//              / 0.75; 80000: Cu 2.23 / 2.66, Au 3.16 / 4.01, Si 0.88 / 0.98;
+//              1e6: Cu 12.6 / 21.5, Au 12.9 / 33.4, Si 5.7 / 8.0)
 //   FP32 continuous, whose lengths differ by backscattering alone: 1e6
-//              electrons Cu 70 deg 2.64 / 4.26, Al 70 deg 1.77 / 2.27, Au 0 deg
+//              electrons Cu 70 deg 2.50 / 4.26, Al 70 deg 1.77 / 2.27, Au 0 deg
 //              7.5 / 10.8, Cu 0 deg 3.97 / 4.30, but Al 0 deg 2.39 / 2.28;
 //              (Cu 70 deg 100000: 0.48 / 0.58, 40000: 0.33 / 0.36, 10000: 0.28
 //              / 0.28)

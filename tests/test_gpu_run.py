@@ -17,9 +17,9 @@ RUNS = {
     "limit": dict(input_par("Si", 5000.0, 1000.0, 0.0), maxScatt=150),
     "cont": dict(input_par("Cu", 10000.0, 1000.0, 70.0, mode="cont", bethe="JL")),
 }
-# one warp per SM partly filled, one wave of 512, the change to 1024, more than
-# one wave of lanes
-SIZES = [70 * SMS, 70 * SMS + 1, 257 * SMS - 3, 512 * SMS, 512 * SMS + 1, 1024 * SMS + 5, 2300 * SMS + 1]
+# one warp per SM partly filled, one wave of 512, the change to 896, one wave of
+# them and more than one
+SIZES = [58 * SMS, 70 * SMS + 1, 257 * SMS - 3, 512 * SMS, 512 * SMS + 1, 896 * SMS, 896 * SMS + 1, 2300 * SMS + 1]
 
 
 @pytest.mark.parametrize("n", SIZES)
