@@ -228,6 +228,17 @@ __global__ void __launch_bounds__(256) k_adj_fwd(const SimConst<T> cp, const Adj
     }
 }
 
+// A positive normal weight as a double (the build flushes subnormals, also in
+// the comparison with zero before the sum).  In FP32 by its bits, as the
+// conversion would hold the FP64 pipe, which bounds the pass, for as long as
+// the addition does: the pass over 1M Cu electrons and 100 bins 80 us with the
+// conversion, 45 us without.
+__device__ __forceinline__ double widen(double x) { return x; }
+__device__ __forceinline__ double widen(float x) {
+    const uint32_t b = __float_as_uint(x);
+    return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+}
+
 // The soft bins, the sum and the number of the backscattered electrons of a
 // forward pass.  A warp reads 32 electrons at a time and takes the
 // backscattered ones in turn, lane l evaluating bins l, l + 32, .. in T and
@@ -267,7 +278,7 @@ __global__ void __launch_bounds__(256) k_adj_bins(const SoftHist sh, const AdjBu
                 if (b >= b0 && b <= b1) {
                     const T d = v - (lo + ((T)b + (T)0.5) * w);
                     const T x = exp(-d * d * i2);
-                    if (x > (T)0) acc[j] += (double)x;
+                    if (x > (T)0) acc[j] += widen(x);
                 }
             }
         }

@@ -22,7 +22,8 @@ namespace mcd {
 constexpr int kThreadsMost = 896;
 
 template <int MODE, bool REC, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_run(const SimConst<float> cp, mcd_tally* tally, const mcd_electron_out eo,
+__global__ void __launch_bounds__(THREADS) k_run(const SimConst<float> cp, const __grid_constant__ RoundKeys keys,
+                                                 mcd_tally* tally, const mcd_electron_out eo,
                                                  const mcd_event_ring ring, uint32_t* status) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ BlockTally bt;
@@ -34,7 +35,7 @@ __global__ void __launch_bounds__(THREADS) k_run(const SimConst<float> cp, mcd_t
     }
     bt_zero(&bt, 1);
     __syncthreads();
-    const HotConst<float> hot(c);
+    const HotConst<float> hot(c, MODE == MCD_MODE_CONT ? &keys : nullptr);
     const OneSim<MODE, HotConst<float>> run{c, hot, bt, tally, rows};
     const unsigned count = (unsigned)(((unsigned long long)c.num_el - blockIdx.x + gridDim.x - 1) / gridDim.x);
     auto take = [&](unsigned k, Lane<float>& L, ElecRng& rng, int& sim) {
@@ -55,10 +56,11 @@ static int launch_threads(const SimConst<float>& c, int sms, mcd_tally* tally, c
                           const mcd_event_ring& ring, uint32_t* status, cudaStream_t st) {
     const unsigned grid = (unsigned)(c.num_el < sms ? c.num_el : sms);
     if (grid == 0) return MCD_OK;
+    const RoundKeys keys = round_keys(c);
     if (c.num_el <= (int64_t)512 * sms)
-        k_run<MODE, REC, 512><<<grid, 512, drain_smem(512), st>>>(c, tally, rows, ring, status);
+        k_run<MODE, REC, 512><<<grid, 512, drain_smem(512), st>>>(c, keys, tally, rows, ring, status);
     else
-        k_run<MODE, REC, kThreadsMost><<<grid, kThreadsMost, drain_smem(kThreadsMost), st>>>(c, tally, rows, ring, status);
+        k_run<MODE, REC, kThreadsMost><<<grid, kThreadsMost, drain_smem(kThreadsMost), st>>>(c, keys, tally, rows, ring, status);
     return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
 }
 
