@@ -376,9 +376,12 @@ typedef struct mcd_softhist {
 
 /* Per-electron adjoint state (device, caller-owned).                         */
 typedef struct mcd_adjoint_buf {
-    void* ckpt;              /* T [max_ckpt][num_el] (exit energy: E every 64
-                                events) or T [max_ckpt][8][num_el] (depth: E,
-                                z, direction and local y axis every 64 events) */
+    void* ckpt;              /* T [max_ckpt][num_el] (exit energy: the first
+                                num_el hold dE_exit/dJ_scale) or
+                                T [max_ckpt][8][num_el] (depth: E, z, direction
+                                and local y axis every 64 events).  An electron
+                                of more than 64 max_ckpt events up to kstar sets
+                                the checkpoint flag and carries no gradient    */
     int32_t* kstar;          /* [num_el], 'bks' electrons, else -1: the exit
                                 event (exit energy) or the number of events
                                 up to the deepest point (depth)              */
@@ -394,7 +397,7 @@ typedef struct mcd_adjoint_buf {
                                 electron instead                            */
 } mcd_adjoint_buf;
 
-/* Continuous-mode forward pass that also stores the adjoint checkpoints.
+/* Continuous-mode forward pass that also stores the adjoint state.
  * hist_out[nbins + 2] (device, zeroed by the caller) receives the unnormalised
  * soft bins of hist->quantity, its sum and the number of 'bks' electrons; tally
  * (may be NULL) the outcome and event counts.  sim->J_scale and sim->n_scale
@@ -405,13 +408,15 @@ int mcd_adjoint_forward(const mcd_sim* sim, const mcd_material* mat, const mcd_s
                         const mcd_adjoint_buf* buf, double* hist_out, mcd_tally* tally,
                         uint32_t* status, void* stream);
 
-/* Reverse sweep: grad_hist[nbins + 1] holds dL/dh_b and dL/d(sum of the
+/* Backward pass: grad_hist[nbins + 1] holds dL/dh_b and dL/d(sum of the
  * quantity); grad[2] (device, zeroed by the caller) receives dL/dJ_scale and
  * dL/dn_scale, the pathwise derivatives with random numbers and event
- * sequence (for depth also the deepest event) frozen.  Each 64-event segment
- * is recomputed from its checkpoint and the Philox counters; for depth the
- * sweep carries the adjoints of the energy, the direction and the local y
- * axis through the Rutherford deflections.  No counterpart in the reference. */
+ * sequence (for depth also the deepest event) frozen, at the parameters of the
+ * forward pass.  The exit energy's derivative was carried along by the forward
+ * pass; for depth each 64-event segment is recomputed from its checkpoint and
+ * the Philox counters, and the adjoints of the energy, the direction and the
+ * local y axis are swept back through the Rutherford deflections.  No
+ * counterpart in the reference. */
 int mcd_adjoint(const mcd_sim* sim, const mcd_material* mat, const mcd_softhist* hist,
                 const mcd_adjoint_buf* buf, const double* grad_hist, double* grad, void* stream);
 

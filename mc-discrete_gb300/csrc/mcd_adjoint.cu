@@ -6,20 +6,23 @@
 // (MC/tools/stoppingPowers.py:112-215).  With the random numbers and the
 // event sequence frozen (the event k* in which an electron leaves through
 // the surface is fixed), the exit energy E_{k*} is a smooth function of the
-// Bethe mean ionisation energy J and of the density n, and its gradient is a
-// scalar reverse sweep along that recursion:
+// Bethe mean ionisation energy J and of the density n.  Its derivative follows
+// the same recursion: with e_k = dE_k/dJ,
 //
-//   lambda_{k*} = dL/dE_exit
-//   dL/dJ      += lambda_{k+1} * (-s_k dS/dJ(E_k))
-//   dL/dn      += lambda_{k+1} * (-(ds_k/dn S + s_k dS/dn))     (= 0: s ~ 1/n, S ~ n)
-//   lambda_k    = lambda_{k+1} * (1 - ds_k/dE S - s_k dS/dE)
+//   e_{k+1} = e_k (1 + s_k (dlnsig/dE S - dS/dE)) - s_k dS/dJ
+//   dL/dJ   = sum over electrons of dL/dE_exit e_{k*};   dL/dn = 0  (s ~ 1/n, S ~ n)
 //
-// The forward kernel runs the full transport (positions and directions decide
-// k*) and stores E every 64 events; the backward kernel recomputes each
-// 64-event segment from its checkpoint and the Philox counters, then sweeps
-// it in reverse.  Tallies are Gaussian-soft bins of the exit energy of
-// backscattered electrons, h_b = (1/N) sum exp(-(E - c_b)^2 / (2 sigma^2)),
-// and the sum of exit energies.
+// For one parameter that is as cheap as the adjoint recursion and needs no
+// event twice: the forward pass carries e along, and the backward pass is one
+// multiplication per electron.  The deepest z instead takes a reverse sweep: its
+// derivative through the rotations grows by orders of magnitude along deep
+// trajectories, so that another order of evaluation in FP32 gives other
+// gradients there.  Its forward pass stores the state every 64 events; the
+// backward pass recomputes each 64-event segment from its checkpoint and the
+// Philox counters, then sweeps it in reverse.  Tallies are Gaussian-soft bins of
+// the exit energy (or deepest z) of backscattered electrons,
+// h_b = (1/N) sum exp(-(q - c_b)^2 / (2 sigma^2)),
+// and their sum.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -30,7 +33,7 @@ namespace mcd {
 constexpr int kSeg = 64;  // events per checkpoint segment
 
 struct AdjBuf {
-    void* ckpt;        // T, max_ckpt x num_el (checkpoint-major)
+    void* ckpt;        // T, [num_el] dE/dJ_scale, or (depth) max_ckpt x 8 x num_el (checkpoint-major)
     int32_t* kstar;    // exit event of 'bks' electrons, -1 otherwise
     void* E_exit;      // T
     int32_t max_ckpt;
@@ -106,13 +109,31 @@ __device__ __forceinline__ void stopping_derivs(const C& c, T E, T* S, T* SE, T*
 // d ln(sigma'_R)/dE
 template <class T, class C>
 __device__ __forceinline__ T dlnsig(const C& c, T E) {
-    const T rel = c.ruth_r2 ? (T)2 * (Ops<T>::div((T)1, E + (T)511000) - Ops<T>::div((T)1, E + (T)1024000))
+    const T rel = (c.bits & kBitR2) ? (T)2 * (Ops<T>::div((T)1, E + (T)511000) - Ops<T>::div((T)1, E + (T)1024000))
                             : (T)0;
     return rel - Ops<T>::div((T)1, E + c.aS);
 }
 
-// The forward pass: every electron's full transport, with its checkpoints
-// every kSeg events.  With a queue word (buf.queue) the grid is resident and
+// dE/dJ_scale after an event of step s and loss dE = s S at the energy E, from
+// its value e before it; ij = 1 / J_scale.  In terms of dE and s bP / E, which
+// the event has computed, the derivatives of s and S take a dozen instructions.
+template <class T, class C>
+__device__ __forceinline__ T tangent(const C& c, T E, T s, T dE, T e, T ij) {
+    const T iE = Ops<T>::div((T)1, E), up = dE * (dlnsig<T>(c, E) + iE);   // s (dlnsig S + S / E)
+    if (c.bethe == MCD_BETHE_CLASSICAL) {
+        const T sb = s * Ops<T>::div(c.bP, E);
+        return e + e * (up - sb * iE) + ij * sb;
+    }
+    if (c.bethe == MCD_BETHE_JL) {
+        const T sb = s * Ops<T>::div(c.bP, E), q = Ops<T>::div((T)1, E + c.bkJ);
+        return e + e * (up - sb * q) + ij * (sb - sb * (c.bkJ * q));
+    }
+    return e + e * (up - s * Ops<T>::div(c.bX, E) * c.bW * iE);
+}
+
+// The forward pass: every electron's full transport, with (exit energy) the
+// derivative of its energy carried along or (depth) its checkpoints every kSeg
+// events.  With a queue word (buf.queue) the grid is resident and
 // a lane that finishes its electron takes the next from the queue, so that
 // lanes do not idle while the longest trajectory of their warp runs (one
 // thread per electron kept about 18 of 32 lanes busy); without one, each
@@ -122,10 +143,14 @@ __device__ __forceinline__ T dlnsig(const C& c, T E) {
 // here a lane or two at a time would evaluate some five bins each and add them
 // to shared FP64 sums by compare-and-swap.  With the constants in registers
 // and one vote per event, forward and backward with their host calls: exit
-// energy of 1e6 electrons 2.97 -> 2.65 ms, depth of 3e5 1.76 -> 1.61 ms.
+// energy of 1e6 Al electrons 2.97 -> 2.65 ms, depth of 3e5 1.76 -> 1.61 ms.  The
+// derivative carried along costs the exit-energy pass 4% (1.69 -> 1.76 ms)
+// and leaves 0.09 of the backward's 0.51 ms: together 2.62 -> 2.22 ms.  Its
+// FP32 error against FP64 along the same events, over 40 parameter sets, is
+// 3.6e-7 rms, the reverse sweep's was 4.0e-7.
 template <class T, bool DEPTH>
 __global__ void __launch_bounds__(256) k_adj_fwd(const SimConst<T> cp, const AdjBuf buf, uint32_t range,
-                                                 mcd_tally* tally, uint32_t* status) {
+                                                 double inv_j, mcd_tally* tally, uint32_t* status) {
     __shared__ SimConst<T> full;
     __shared__ unsigned long long s_cnt[9];
     if (threadIdx.x == 0) full = cp;
@@ -147,6 +172,8 @@ __global__ void __launch_bounds__(256) k_adj_fwd(const SimConst<T> cp, const Adj
     bool have = false;
     int mstar = 0;   // (depth) events up to the deepest point
     T zbest = (T)0;
+    const T ij = (T)inv_j;
+    T tan = (T)0;    // (exit energy) dE/dJ_scale
     while (true) {
         // the lanes without an electron; voted again only after a refill
         unsigned idle = __ballot_sync(0xffffffffu, !have);
@@ -167,6 +194,8 @@ __global__ void __launch_bounds__(256) k_adj_fwd(const SimConst<T> cp, const Adj
                 if (DEPTH) {
                     mstar = 0;
                     zbest = (T)0;
+                } else {
+                    tan = (T)0;
                 }
                 have = true;
             }
@@ -178,37 +207,37 @@ __global__ void __launch_bounds__(256) k_adj_fwd(const SimConst<T> cp, const Adj
             continue;
         }
         if (!have) continue;
-        if ((L.step % kSeg) == 0) {
+        if (DEPTH && (L.step % kSeg) == 0) {
             const int64_t m = L.step / kSeg;
             if (m < buf.max_ckpt) {
-                if constexpr (!DEPTH) {
-                    ck[(size_t)m * n + i] = L.E;
-                } else {
-                    T* q = ck + (size_t)m * kDepthState * n + i;
-                    q[0] = L.E;
-                    q[n] = L.z;
-                    q[2 * n] = L.dx;
-                    q[3 * n] = L.dy;
-                    q[4 * n] = L.dz;
-                    q[5 * n] = L.yx;
-                    q[6 * n] = L.yy;
-                    q[7 * n] = L.yz;
-                }
+                T* q = ck + (size_t)m * kDepthState * n + i;
+                q[0] = L.E;
+                q[n] = L.z;
+                q[2 * n] = L.dx;
+                q[3 * n] = L.dy;
+                q[4 * n] = L.dz;
+                q[5 * n] = L.yx;
+                q[6 * n] = L.yy;
+                q[7 * n] = L.yz;
             }
         }
-        EventOut<T> ev;
-        cont_event<T, false>(L, c, rng, &ev);
+        EventOut<T> ev;   // (exit energy) the event's E and step; the rest is not stored
+        cont_event<T, !DEPTH>(L, c, rng, &ev);
         if (DEPTH && L.max_z > zbest) {
             zbest = L.max_z;
             mstar = (int)L.step;
         }
-        if (L.outcome == MCD_OUT_NONE) continue;
+        if (L.outcome == MCD_OUT_NONE) {
+            if constexpr (!DEPTH) tan = tangent<T>(c, ev.E, ev.pathl, ev.W, tan, ij);
+            continue;
+        }
         // the electron is done; a 'bks' one left in its last event
         const bool bks = L.outcome == MCD_OUT_BKS;
         const int key = DEPTH ? mstar : (int)(L.step - 1);
         if (bks && key > 0 && (key - 1) / kSeg >= buf.max_ckpt) st |= MCD_FLAG_CKPT;
         buf.kstar[i] = bks ? key : -1;
         static_cast<T*>(buf.E_exit)[i] = DEPTH ? L.max_z : L.E_row;
+        if (!DEPTH) ck[i] = tan;
         if (tally) {
             atomicAdd(&s_cnt[L.outcome & 7], 1ull);
             atomicAdd(&s_cnt[8], (unsigned long long)L.step);
@@ -299,7 +328,7 @@ __global__ void __launch_bounds__(256) k_adj_bins(const SoftHist sh, const AdjBu
 
 template <class T>
 static void launch_bins(const SoftHist& sh, const AdjBuf& ab, int64_t n, int sms, double* hout, cudaStream_t st) {
-    const int64_t blocks = (n + 255) / 256, cap = 4ll * (sms > 0 ? sms : 1);
+    const int64_t blocks = (n + 255) / 256, cap = 4ll * sms;
     const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
     if (sh.nbins <= 32) k_adj_bins<T, 1><<<grid, 256, 0, st>>>(sh, ab, n, hout);
     else if (sh.nbins <= 64) k_adj_bins<T, 2><<<grid, 256, 0, st>>>(sh, ab, n, hout);
@@ -421,8 +450,8 @@ __device__ __forceinline__ void depth_segment(const C& c, const AdjBuf& buf, uin
     A = DepthAdj<T>{lE, ldx, ldy, ldz, lyx, lyy, lyz, sj, sn};
 }
 
-// The backward pass runs only for backscattered electrons, a fraction of
-// the launch: each warp owns a range of kBwdRange electrons and hands its
+// The depth's backward pass runs only for backscattered electrons, a fraction
+// of the launch: each warp owns a range of kBwdRange electrons and hands its
 // backscattered ones to idle lanes in index order, so that warps stay full
 // (one thread per electron left about 5 of 32 lanes active).
 constexpr int kBwdRange = 256;
@@ -479,10 +508,27 @@ __device__ __forceinline__ T exit_adjoint(const SoftHist& sh, const AdjBuf& buf,
     return g;
 }
 
-template <class T, bool DEPTH>
-__global__ void __launch_bounds__(128, 8) k_adj_bwd(const SimConst<T> cp, const SoftHist sh, const AdjBuf buf,
-                                                 const double* grad_h, double inv_n, double inv_j,
-                                                 double inv_ns, double* grad) {
+// Adds the threads' sums to grad; called by the whole block, red[2] zeroed
+__device__ __forceinline__ void add_grad(double* red, double dj, double dn, double* grad) {
+    for (int o = 16; o > 0; o >>= 1) {
+        dj += __shfl_down_sync(0xffffffffu, dj, o);
+        dn += __shfl_down_sync(0xffffffffu, dn, o);
+    }
+    if ((threadIdx.x & 31u) == 0) {
+        atomicAdd(&red[0], dj);
+        atomicAdd(&red[1], dn);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicAdd(&grad[0], red[0]);
+        atomicAdd(&grad[1], red[1]);
+    }
+}
+
+template <class T>
+__global__ void __launch_bounds__(128, 8) k_adj_depth(const SimConst<T> cp, const SoftHist sh, const AdjBuf buf,
+                                                      const double* grad_h, double inv_n, double inv_j,
+                                                      double inv_ns, double* grad) {
     __shared__ SimConst<T> c;
     __shared__ double red[2];
     __shared__ T gh[MCD_HIST_E_MAX + 1];
@@ -497,17 +543,16 @@ __global__ void __launch_bounds__(128, 8) k_adj_bwd(const SimConst<T> cp, const 
     const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint64_t lo = warp * (uint64_t)kBwdRange;
     BksFeed f{lo < n ? lo : n, lo + kBwdRange < n ? lo + kBwdRange : n, 0, 0u};
-    const T* ck = static_cast<const T*>(buf.ckpt);
     // the lane's sums over its electrons, in T (a few electrons per lane),
     // and over the lanes and blocks in FP64
     T gj = (T)0, gn = (T)0;
-    // lane state: its electron, the exit event, the segment to sweep next and
-    // (exit energy) the adjoint of E and the electron's parameter sums
+    // lane state: its electron, the events up to the deepest point, the segment to sweep next,
+    // g = dL/dZ and the adjoints carried between segments
     int64_t cur = -1;
     ElecRng rng{0u, 0u, 0u};
     int ks = 0, m = 0;
-    T lam = (T)0, sj = (T)0, sn = (T)0;
-    DepthAdj<T> dA{};   // depth: the adjoints carried between segments
+    T g = (T)0;
+    DepthAdj<T> dA{};
     const T ij = (T)inv_j, ins = (T)inv_ns;
     while (true) {
         const unsigned idle = __ballot_sync(0xffffffffu, cur < 0);
@@ -518,65 +563,54 @@ __global__ void __launch_bounds__(128, 8) k_adj_bwd(const SimConst<T> cp, const 
                 rng = elec_rng(c, c.first + (uint64_t)e);
                 ks = buf.kstar[e];
                 m = (ks - 1) / kSeg;
-                // the sweep runs in the transport precision: lambda is a
-                // product of factors 1 + O(1e-2) and each step adds one term
-                lam = exit_adjoint<T>(sh, buf, gh, (uint64_t)e);
-                sj = sn = (T)0;
-                if constexpr (DEPTH) dA = DepthAdj<T>{};
+                g = exit_adjoint<T>(sh, buf, gh, (uint64_t)e);
+                dA = DepthAdj<T>{};
             }
         }
         if (__ballot_sync(0xffffffffu, cur >= 0) == 0u) break;
         if (cur < 0) continue;
-        const uint64_t i = (uint64_t)cur;
-        if constexpr (DEPTH) {   // one segment per trip; lam holds g = dL/dZ
-            depth_segment<T>(c, buf, i, rng, ks, m, lam, ij, ins, dA);
-            if (--m < 0) {
-                gj += dA.sj;
-                gn += dA.sn;
-                cur = -1;
-            }
-            continue;
-        }
-        // exit energy: one 64-event segment per trip, the last one first
-        const int k0 = m * kSeg;
-        const int len = min(kSeg, ks - k0);
-        T Eseg[kSeg], sseg[kSeg];
-        T E = ck[(size_t)m * n + i];
-        for (int j = 0; j < len; ++j) {   // recompute the segment exactly as the forward did
-            const T s = step_len<T>(c, E, rng, k0 + j);
-            Eseg[j] = E;
-            sseg[j] = s;
-            E = E - Ops<T>::mul_rn(s, stopping<T>(c, E));
-        }
-        for (int j = len - 1; j >= 0; --j) {   // reverse sweep
-            const T Ek = Eseg[j], s = sseg[j];
-            T S, SE, Sj;
-            stopping_derivs<T>(c, Ek, &S, &SE, &Sj);
-            sj += lam * (-s * Sj * ij);
-            // ds/dn = -s/n and dS/dn = S/n: the two terms cancel
-            sn += lam * (-((-s * ins) * S + s * (S * ins)));
-            lam *= (T)1 + s * (dlnsig<T>(c, Ek) * S - SE);
-        }
+        // one segment per trip, the last one first
+        depth_segment<T>(c, buf, (uint64_t)cur, rng, ks, m, g, ij, ins, dA);
         if (--m < 0) {
-            gj += sj;
-            gn += sn;
+            gj += dA.sj;
+            gn += dA.sn;
             cur = -1;
         }
     }
-    double dj = (double)gj, dn = (double)gn;
-    for (int o = 16; o > 0; o >>= 1) {
-        dj += __shfl_down_sync(0xffffffffu, dj, o);
-        dn += __shfl_down_sync(0xffffffffu, dn, o);
-    }
-    if (lane == 0) {
-        atomicAdd(&red[0], dj);
-        atomicAdd(&red[1], dn);
-    }
+    add_grad(red, (double)gj, (double)gn, grad);
+}
+
+// The exit energy's gradient: every backscattered electron's dL/dE_exit times
+// the derivative that the forward pass left.  It reads 8 to 12 bytes per
+// electron and evaluates the few bins in reach.  Sums in FP64; the density does
+// not enter the exit energy (s ~ 1/n, S ~ n), and its sum shows only a gradient
+// that is not finite.
+template <class T>
+__global__ void __launch_bounds__(256) k_adj_exit(const SoftHist sh, const AdjBuf buf, int64_t n, const double* grad_h,
+                                                  double inv_n, double* grad) {
+    __shared__ double red[2];
+    __shared__ T gh[MCD_HIST_E_MAX + 1];
+    if (threadIdx.x < 2) red[threadIdx.x] = 0.0;
+    for (int b = threadIdx.x; b <= sh.nbins; b += blockDim.x) gh[b] = (T)(b < sh.nbins ? grad_h[b] * inv_n : grad_h[b]);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        atomicAdd(&grad[0], red[0]);
-        atomicAdd(&grad[1], red[1]);
+    const T* ck = static_cast<const T*>(buf.ckpt);
+    double gj = 0.0, gn = 0.0;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const int k = buf.kstar[i];
+        if (k <= 0 || (k - 1) / kSeg >= buf.max_ckpt) continue;
+        const T g = exit_adjoint<T>(sh, buf, gh, (uint64_t)i);
+        gj += (double)(g * ck[i]);
+        gn += (double)(g * (T)0);
     }
+    __syncwarp();
+    add_grad(red, gj, gn, grad);
+}
+
+template <class T>
+static void launch_exit(const SoftHist& sh, const AdjBuf& ab, int64_t n, int sms, const double* grad_h, double inv_n,
+                        double* grad, cudaStream_t st) {
+    const int64_t blocks = (n + 255) / 256, cap = 8ll * sms;
+    k_adj_exit<T><<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, st>>>(sh, ab, n, grad_h, inv_n, grad);
 }
 
 // E_{k*}(J, n) along the frozen event sequence only (no geometry): the
@@ -620,6 +654,15 @@ __global__ void __launch_bounds__(256) k_adj_chain(const SimConst<T> cp, const S
     __syncthreads();
     for (int b = threadIdx.x; b < sh.nbins + 2; b += blockDim.x)
         if (sh_h[b] != 0.0) atomicAdd(&hout[b], sh_h[b]);
+}
+
+// multiprocessors of the current device, 0 on an error
+static int sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return sms;
 }
 
 static int adj_args(const mcd_sim* sim, const mcd_material* mat, const mcd_softhist* hist,
@@ -671,10 +714,9 @@ extern "C" int mcd_adjoint_forward(const mcd_sim* sim, const mcd_material* mat, 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const uint32_t range = 32;
     unsigned long long grid = ((unsigned long long)sim->num_el + 255) / 256;   // one thread per electron
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return MCD_ECUDA;
+    const int sms = sm_count();
+    if (sms <= 0) return MCD_ECUDA;
+    const double inv_j = 1.0 / (sim->J_scale > 0 ? sim->J_scale : 1.0);
     const bool depth = sh.quantity == MCD_ADJ_MAX_DEPTH, fp64 = sim->precision == MCD_FP64;
     const void* kern = fp64 ? (depth ? (const void*)k_adj_fwd<double, true> : (const void*)k_adj_fwd<double, false>)
                             : (depth ? (const void*)k_adj_fwd<float, true> : (const void*)k_adj_fwd<float, false>);
@@ -683,7 +725,7 @@ extern "C" int mcd_adjoint_forward(const mcd_sim* sim, const mcd_material* mat, 
         // more than there are electrons for
         int blocks = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, 256, 0) != cudaSuccess) return MCD_ECUDA;
-        const unsigned long long resident = (unsigned long long)(sms > 0 ? sms : 1) * (blocks > 0 ? blocks : 1);
+        const unsigned long long resident = (unsigned long long)sms * (blocks > 0 ? blocks : 1);
         grid = grid < resident ? grid : resident;
         if (cudaMemsetAsync(ab.queue, 0, sizeof(unsigned long long), st) != cudaSuccess) return MCD_ECUDA;
     }
@@ -691,14 +733,14 @@ extern "C" int mcd_adjoint_forward(const mcd_sim* sim, const mcd_material* mat, 
     const unsigned g = (unsigned)grid;
     if (fp64) {
         const SimConst<double> c = make_consts<double>(*sim, *mat, nullptr, nullptr);
-        if (depth) k_adj_fwd<double, true><<<g, 256, 0, st>>>(c, ab, range, tally, status);
-        else k_adj_fwd<double, false><<<g, 256, 0, st>>>(c, ab, range, tally, status);
+        if (depth) k_adj_fwd<double, true><<<g, 256, 0, st>>>(c, ab, range, inv_j, tally, status);
+        else k_adj_fwd<double, false><<<g, 256, 0, st>>>(c, ab, range, inv_j, tally, status);
         if (cudaGetLastError() != cudaSuccess) return MCD_ECUDA;
         launch_bins<double>(sh, ab, sim->num_el, sms, hist_out, st);
     } else {
         const SimConst<float> c = make_consts<float>(*sim, *mat, nullptr, nullptr);
-        if (depth) k_adj_fwd<float, true><<<g, 256, 0, st>>>(c, ab, range, tally, status);
-        else k_adj_fwd<float, false><<<g, 256, 0, st>>>(c, ab, range, tally, status);
+        if (depth) k_adj_fwd<float, true><<<g, 256, 0, st>>>(c, ab, range, inv_j, tally, status);
+        else k_adj_fwd<float, false><<<g, 256, 0, st>>>(c, ab, range, inv_j, tally, status);
         if (cudaGetLastError() != cudaSuccess) return MCD_ECUDA;
         launch_bins<float>(sh, ab, sim->num_el, sms, hist_out, st);
     }
@@ -712,28 +754,28 @@ extern "C" int mcd_adjoint(const mcd_sim* sim, const mcd_material* mat, const mc
     int rc = adj_args(sim, mat, hist, buf, &sh, &ab);
     if (rc != MCD_OK) return rc;
     if (!grad_hist || !grad) return MCD_EINVAL;
+    if (sim->num_el == 0) return MCD_OK;
+    const double inv_n = 1.0 / (double)sim->num_el;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (sh.quantity != MCD_ADJ_MAX_DEPTH) {
+        const int sms = sm_count();
+        if (sms <= 0) return MCD_ECUDA;
+        if (sim->precision == MCD_FP64) launch_exit<double>(sh, ab, sim->num_el, sms, grad_hist, inv_n, grad, st);
+        else launch_exit<float>(sh, ab, sim->num_el, sms, grad_hist, inv_n, grad, st);
+        return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
+    }
     // one warp per kBwdRange electrons, four warps per block
     const unsigned long long grid = ((unsigned long long)sim->num_el + 4 * kBwdRange - 1) / (4 * kBwdRange);
-    if (grid == 0) return MCD_OK;
     if (grid > 0x7fffffffull) return MCD_ETOOBIG;
-    const double inv_n = 1.0 / (double)sim->num_el;
     const double js = 1.0 / (sim->J_scale > 0 ? sim->J_scale : 1.0);
     const double ns = 1.0 / (sim->n_scale > 0 ? sim->n_scale : 1.0);
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool depth = sh.quantity == MCD_ADJ_MAX_DEPTH;
-    if (sim->precision == MCD_FP64) {
-        const SimConst<double> c = make_consts<double>(*sim, *mat, nullptr, nullptr);
-        if (depth)
-            k_adj_bwd<double, true><<<(unsigned)grid, 128, 0, st>>>(c, sh, ab, grad_hist, inv_n, js, ns, grad);
-        else
-            k_adj_bwd<double, false><<<(unsigned)grid, 128, 0, st>>>(c, sh, ab, grad_hist, inv_n, js, ns, grad);
-    } else {
-        const SimConst<float> c = make_consts<float>(*sim, *mat, nullptr, nullptr);
-        if (depth)
-            k_adj_bwd<float, true><<<(unsigned)grid, 128, 0, st>>>(c, sh, ab, grad_hist, inv_n, js, ns, grad);
-        else
-            k_adj_bwd<float, false><<<(unsigned)grid, 128, 0, st>>>(c, sh, ab, grad_hist, inv_n, js, ns, grad);
-    }
+    const unsigned g = (unsigned)grid;
+    if (sim->precision == MCD_FP64)
+        k_adj_depth<double><<<g, 128, 0, st>>>(make_consts<double>(*sim, *mat, nullptr, nullptr), sh, ab, grad_hist,
+                                               inv_n, js, ns, grad);
+    else
+        k_adj_depth<float><<<g, 128, 0, st>>>(make_consts<float>(*sim, *mat, nullptr, nullptr), sh, ab, grad_hist,
+                                              inv_n, js, ns, grad);
     return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
 }
 

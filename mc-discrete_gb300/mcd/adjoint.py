@@ -1,9 +1,9 @@
 """Differentiable continuous-mode transport.
 
 ExitEnergyModel runs the continuous-slowing-down transport (mcd_adjoint_forward)
-and keeps, per electron, checkpoints every 64 events.  Its backward pass
-(mcd_adjoint) recomputes each 64-event segment from the Philox counters and
-sweeps it in reverse, giving the pathwise derivatives of
+and keeps, per electron, the derivative of its exit energy or (depth) its state
+every 64 events.  The backward pass (mcd_adjoint) gives the pathwise derivatives
+of
 
     h_b = (1/N) sum_{bks} exp(-(q - c_b)^2 / (2 sigma^2))   (b < nbins)
     m   = mean of q over backscattered electrons
@@ -57,7 +57,7 @@ class ExitEnergyModel:
         self.nbins = int(nbins)
         self.max_ckpt = int(max_ckpt)
         self._alloc()
-        self.last = None   # (J_scale, n_scale) of the stored checkpoints
+        self.last = None   # (J_scale, n_scale) of the last forward pass
 
     def _alloc(self):
         torch = _torch()
