@@ -186,16 +186,18 @@ constexpr CxDD cx_div(CxDD x, double d) {   // x / d
     const double q2 = ((r.hi + r.lo) - p.lo + x.lo) / d;
     return cx_two_sum(q1, q2);
 }
-// ln(1 + j/256) = 2 atanh(y), y = j / (512 + j) < 1/3
-constexpr double cx_ln_ratio(int j) {
-    const CxDD y = cx_div(CxDD{(double)j, 0.0}, 512.0 + j), y2 = cx_mul(y, y);
+// 2 atanh(a / d) by n terms of its series
+constexpr CxDD cx_atanh2(double a, double d, int n) {
+    const CxDD y = cx_div(CxDD{a, 0.0}, d), y2 = cx_mul(y, y);
     CxDD term = y, sum{0.0, 0.0};
-    for (int k = 0; k < 36; ++k) {
+    for (int k = 0; k < n; ++k) {
         sum = cx_add(sum, cx_div(term, 2.0 * k + 1.0));
         term = cx_mul(term, y2);
     }
-    return 2.0 * sum.hi + 2.0 * sum.lo;
+    return CxDD{2.0 * sum.hi, 2.0 * sum.lo};
 }
+// ln(1 + j/256) = 2 atanh(y), y = j / (512 + j) < 1/3
+constexpr CxDD cx_ln_ratio(int j) { return cx_atanh2((double)j, 512.0 + j, 36); }
 struct CxPair {
     double s, c;
 };
@@ -216,7 +218,7 @@ constexpr CxPair cx_sincos(int a) {
 constexpr F64Tabs cx_f64_tabs() {
     F64Tabs t{};
     for (int j = 0; j < 256; ++j) {
-        t.lnm[j] = cx_ln_ratio(j);
+        t.lnm[j] = cx_ln_ratio(j).hi + cx_ln_ratio(j).lo;
         t.invm[j] = 256.0 / (256.0 + j);
         // reduce to [0, pi/4]: sin(pi - x) = sin x, cos(pi - x) = -cos x;
         // sin(pi/2 - x) = cos x, cos(pi/2 - x) = sin x
