@@ -122,10 +122,6 @@ int launch_lanes(const SimConst<T>& c, int group, mcd_tally* tally, const ElOut&
     switch (group) {
         case 32: return launch_mode<T, 32>(c, tally, eo, ring, rec, status, st);
         case 16: return launch_mode<T, 16>(c, tally, eo, ring, rec, status, st);
-#ifdef TUNE_G
-        case 4: return launch_mode<T, 4>(c, tally, eo, ring, rec, status, st);
-        case 2: return launch_mode<T, 2>(c, tally, eo, ring, rec, status, st);
-#endif
         default: return launch_mode<T, 8>(c, tally, eo, ring, rec, status, st);
     }
 }
