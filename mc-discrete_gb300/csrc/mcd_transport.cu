@@ -313,8 +313,10 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
 
 // The electrons that a batched launch listed, to their end: block b of the
 // grid takes every gridDim.x-th of them, so that each SM gets its part of
-// every simulation's.
-template <bool REC>
+// every simulation's.  ONE: the batch has one simulation, whose constants, in
+// DS mode, stay in registers (40000 Au 30 keV electrons 4.63 -> 4.05 ms, with
+// every event to the ring 6.14 -> 5.94 ms).
+template <bool REC, bool ONE>
 __global__ void __launch_bounds__(kDrainThreads) k_rundown(uint8_t* ws, mcd_tally* tallies, uint32_t* status,
                                                            const mcd_event_ring ring, int flags) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -324,6 +326,7 @@ __global__ void __launch_bounds__(kDrainThreads) k_rundown(uint8_t* ws, mcd_tall
     if (blockIdx.x >= live) return;
     const BatchShared sh(smem, nsims);
     sh.load(ws, nsims);
+    __syncthreads();
     const ManySims run{sh.c, sh.t, tallies, reinterpret_cast<const mcd_electron_out*>(ws + batch_elout_off(nsims))};
     const Seats list{reinterpret_cast<uint32_t*>(ws + batch_live_off(nsims)), kLiveSeats};
     const unsigned count = (live - blockIdx.x + gridDim.x - 1) / gridDim.x;
@@ -332,8 +335,16 @@ __global__ void __launch_bounds__(kDrainThreads) k_rundown(uint8_t* ws, mcd_tall
     };
     uint8_t* seats = smem + batch_drain_off(nsims);
     const bool inl = (flags & kRunInline) != 0;
-    const uint32_t st = hdr->chan ? drain_run<REC, true>(run, count, take, seats, ring, inl)
-                                  : drain_run<REC, false>(run, count, take, seats, ring, inl);
+    uint32_t st;
+    if (ONE && !(sh.c[0].bits & kBitCont)) {
+        const HotConst<float> hot(sh.c[0]);
+        const OneSim<MCD_MODE_DS, HotConst<float>> one{sh.c[0], hot, sh.t[0], tallies, run.rows(0)};
+        st = hdr->chan ? drain_run<REC, true>(one, count, take, seats, ring, inl)
+                       : drain_run<REC, false>(one, count, take, seats, ring, inl);
+    } else {
+        st = hdr->chan ? drain_run<REC, true>(run, count, take, seats, ring, inl)
+                       : drain_run<REC, false>(run, count, take, seats, ring, inl);
+    }
     or_status(status, st);
     __syncthreads();
     sh.flush(tallies, nsims);
@@ -771,13 +782,14 @@ static int launch_batched(void* workspace, int nsims, mcd_tally* tallies, const 
     if (fit < 1) return MCD_ETOOBIG;
     if (per_sm <= 0 || per_sm > fit) per_sm = fit;
     if ((long long)sms * per_sm * block <= kLiveSeats && smem2 + 1024 <= (size_t)most) flags |= kRunList;
-    if ((flags & kRunList) && set_smem(k_rundown<REC>, smem2) != MCD_OK) return MCD_ECUDA;
+    auto down = nsims == 1 ? k_rundown<REC, true> : k_rundown<REC, false>;
+    if ((flags & kRunList) && set_smem(down, smem2) != MCD_OK) return MCD_ECUDA;
     // reset the queue and the list (the first two words of the workspace)
     if (cudaMemsetAsync(workspace, 0, 2 * sizeof(unsigned long long), st) != cudaSuccess) return MCD_ECUDA;
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     kern<<<sms * per_sm, block, smem, st>>>(ws, tallies, refill, status, ring, flags);
     if (cudaGetLastError() != cudaSuccess) return MCD_ECUDA;
-    if (flags & kRunList) k_rundown<REC><<<sms, kDrainThreads, smem2, st>>>(ws, tallies, status, ring, flags);
+    if (flags & kRunList) down<<<sms, kDrainThreads, smem2, st>>>(ws, tallies, status, ring, flags);
     return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
 }
 
