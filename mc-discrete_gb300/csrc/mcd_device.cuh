@@ -286,18 +286,18 @@ __device__ __forceinline__ void cossin2pi_word(uint32_t w, double* c, double* s)
 }
 
 // 1/d for a positive normal d: the hardware approximation
-// (rcp.approx.ftz.f64) refined by two steps of the third-order
-// Newton-Raphson iteration r <- r (1 + e + e^2), e = 1 - d r, which cubes
-// the relative error each step (from any start better than 2^-8 to below
-// 2^-72), so the result is within the rounding of its last operations, two
-// ulp; four FMAs instead of the correctly rounded division's sequence.
+// (rcp.approx.ftz.f64) refined by a third-order step of the Newton-Raphson
+// iteration, r <- r (1 + e + e^2), e = 1 - d r, which cubes the relative error,
+// and a second-order one, which squares it (from any start better than 2^-9 to
+// below 2^-54), so the result is within the rounding of its last operations, two
+// ulp; five FP64 instructions instead of the correctly rounded division's
+// sequence.
 __device__ __forceinline__ double rcp_pos(double d) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
     double e = fma(-d, r, 1.0);
     r = fma(r, fma(e, e, e), r);
-    e = fma(-d, r, 1.0);
-    return fma(r, fma(e, e, e), r);
+    return fma(r, fma(-d, r, 1.0), r);
 }
 
 // |x| by clearing the sign bit (an integer operation, not an FP64 one)

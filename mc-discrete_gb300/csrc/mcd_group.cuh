@@ -143,17 +143,61 @@ struct GroupLanes {
         : t(lane & (G - 1)), h0(lane & ~(G - 1)), gmask(ones << (lane & ~(G - 1))) {}
 };
 
+// The direction update that an FP64 event leaves to group_turn
+template <class T>
+struct GroupTurn {
+    T s2;
+    bool due;
+};
+
+// lane_rotate_cs by the lanes of a group, called by the whole warp: lane q of
+// the first six computes component q mod 3 of the new direction (q < 3) or of
+// the new y axis with the operations of lane_rotate_cs in their order, and
+// every lane of the group receives all six.  The FP64 pipe takes 16 cycles for
+// a warp instruction and a small run's warps share it, so 25 of the event's 77
+// FP64 instructions (35 of the update become 10) are time, and the shuffles
+// that come instead are not: 1000 Si 10 keV electrons 2.51 -> 2.13
+// ms, 700 Au 20 keV 9.8 -> 8.0, 3000 Si 3.7 -> 3.2 (with their host calls).
+template <int G>
+__device__ __forceinline__ void group_turn(Lane<double>& L, const GroupTurn<double>& turn, double cph, double sph,
+                                           const GroupLanes<G>& g) {
+    const double s2 = turn.s2, sth = 2.0 * Ops<double>::sqrt_(s2 * (1.0 - s2)), cth = 1.0 - 2.0 * s2;
+    const double a = sth * cph, b = sth * sph;
+    const int q = g.t % 6, i = q % 3;
+    const bool axis = q >= 3;
+    auto pick = [](int k, double x, double y, double z) { return k == 0 ? x : k == 1 ? y : z; };
+    const double d0 = pick(i, L.dx, L.dy, L.dz), d1 = pick(i, L.dy, L.dz, L.dx), d2 = pick(i, L.dz, L.dx, L.dy);
+    const double y0 = pick(i, L.yx, L.yy, L.yz), y1 = pick(i, L.yy, L.yz, L.yx), y2 = pick(i, L.yz, L.yx, L.yy);
+    const double x = fma(y1, d2, -(y2 * d1));
+    const double v = fma(y0, axis ? 0.0 : b, fma(axis ? y0 : d0, axis ? cph : cth, x * (axis ? -sph : a)));
+    const int src = g.h0 + (axis ? 3 : 0);
+    const double u0 = __shfl_sync(0xffffffffu, v, src), u1 = __shfl_sync(0xffffffffu, v, src + 1),
+                 u2 = __shfl_sync(0xffffffffu, v, src + 2);
+    const double w = v * Ops<double>::renorm(fma(u2, u2, fma(u0, u0, u1 * u1)));
+    double n[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) n[k] = __shfl_sync(0xffffffffu, w, g.h0 + k);
+    if (!turn.due) return;
+    L.dx = n[0];
+    L.dy = n[1];
+    L.dz = n[2];
+    L.yx = n[3];
+    L.yy = n[4];
+    L.yz = n[5];
+}
+
 constexpr int kGroupNone = -1;    // the group took no event (no electron, or at the event limit)
 constexpr int kGroupPlain = -2;   // a Rutherford event that stays in the sample
 
-// One DS event of every group of a warp (called by all its lanes; active: the
+// One DS event of every group of a warp, but in FP64 for its direction update
+// (called by all its lanes; active: the
 // group has an electron; cur: its event's values computed ahead).  Returns the
 // channel code, kGroupNone or kGroupPlain; the step counter has advanced
 // unless it is kGroupNone.
 template <class T, bool REC, int G, class C>
 __device__ __forceinline__ int group_event(Lane<T>& L, GroupSig<T, G>& sig, const C& c, const EventPre<T>& cur,
                                            bool active, uint32_t limit, const GroupLanes<G>& g, T zmax, bool use_tab,
-                                           EventOut<T>* ev) {
+                                           EventOut<T>* ev, GroupTurn<T>* turn = nullptr) {
     // the columns passed: 0 Rutherford, 1 Moller, 2.. Gryz, K-1 Quinn
     const T level = cur.ux * sig.all;
     unsigned below = 0;
@@ -220,7 +264,12 @@ __device__ __forceinline__ int group_event(Lane<T>& L, GroupSig<T, G>& sig, cons
     if (REC) event_out<T>(*ev, L, E, W, path, s2, cur.rw, ch);
     lane_move(L, c, path, ch == MCD_CH_DIFF);
     if (loss && (L.outcome == MCD_OUT_NONE || (c.bits & MCD_Q_CROSSING_STEP))) lane_lose(L, c, W);
-    if (L.outcome == MCD_OUT_NONE) lane_rotate_cs(L, s2, cur.cph, cur.sph);
+    if constexpr (sizeof(T) == 8) {
+        turn->s2 = s2;
+        turn->due = L.outcome == MCD_OUT_NONE;
+    } else if (L.outcome == MCD_OUT_NONE) {
+        lane_rotate_cs(L, s2, cur.cph, cur.sph);
+    }
     return ch;
 }
 

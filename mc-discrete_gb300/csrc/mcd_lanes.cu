@@ -71,7 +71,12 @@ __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst
         EventOut<T> ev;
         int ch = kGroupNone;
         if (MODE == MCD_MODE_DS) {
-            ch = group_event<T, REC, G>(L, sig, c, cur, active, w.w, g, zmax, use_tab, &ev);
+            GroupTurn<T> turn{(T)0, false};
+            ch = group_event<T, REC, G>(L, sig, c, cur, active, w.w, g, zmax, use_tab, &ev, &turn);
+            if constexpr (sizeof(T) == 8) {
+                if (G < 32) __syncwarp();
+                group_turn<G>(L, turn, cur.cph, cur.sph, g);
+            }
         } else if (active) {
             if (step >= w.w) {
                 lane_long(L);

@@ -536,11 +536,15 @@ static int dispatch_plain(const SimConst<T>& c, int block, mcd_tally* tally, con
 //   0.85, 4500 0.95 / 1.08, 7500 1.21 / 1.23, 10000 1.36 / 1.32)
 //   FP32 continuous      1500: 0.21 / 0.23 with 32 / 8;  2500: 0.28 / 0.24;
 //                        4500: 0.25 / 0.27 with 8 / 0;  6500: 0.28 / 0.28
-//   FP64 DS (Si, table)  700: 2.27 / 2.38 with 32 / 16;  1500: 2.65 / 2.66 with
-//                        16 / 8;  3500: 3.48 / 4.35 with 8 / 0;  5000: 4.96 / 4.76
-//   without a table      Si 5000: 13.3 / 14.7 with 8 / 0, 7500 19.7 / 15.3;
-//                        Au 14000: 33 / 66 (the plain kernel evaluates a
-//                        cross section per shell in every event)
+//   FP64 DS (with their host calls; Si, table)  1000: 2.35 / 2.33 with 32 / 16,
+//                        1300: 2.57 / 2.36;  1800: 2.56 / 2.70 with 16 / 8, 2500:
+//                        4.17 / 3.15;  6500: 4.88 / 5.35 with 8 / 0, 7500: 5.56 / 5.34
+//   (Au: 1000 7.98 / 8.69 with 32 / 16, 1300 9.24 / 8.90, 1800 9.21 / 9.76 with
+//   16 / 8, 2500 10.5 / 10.1, 9000 21.2 / 26.3 with 8 / 0)
+//   without a table      Si 7000: 15.7 / 16.5 with 8 / 0, 9000 19.9 / 16.7; Cu
+//                        9000: 25.4 / 29.8, 11000 35.3 / 29.0; Au 14000: 63 / 116
+//                        (the plain kernel evaluates a cross section per
+//                        shell in every event)
 //   FP64 continuous      300: 3.69 / 3.81 with 32 / 8;  1500: 3.99 / 4.55 with 8
 //                        / 0;  2500: 4.72 / 4.54
 static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) {
@@ -550,8 +554,8 @@ static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) 
         return e < 20 ? 32 : e < 33 ? 16 : e < 58 ? 8 : 0;
     }
     if (s.mode != MCD_MODE_DS) return e < 3 ? 32 : e < 10 ? 8 : 0;
-    const int most = s.sigma_table ? 28 : 12 * (m.n_shells > 3 ? m.n_shells : 3);
-    return e < 5 ? 32 : e < 10 ? 16 : e < most ? 8 : 0;
+    const int most = s.sigma_table ? 47 : 16 * (m.n_shells > 3 ? m.n_shells : 3);
+    return e < 7 ? 32 : e < 12 ? 16 : e < most ? 8 : 0;
 }
 
 // Does an automatic run of a thread per electron take one resident block per
