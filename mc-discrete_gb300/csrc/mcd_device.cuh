@@ -970,11 +970,12 @@ __device__ __forceinline__ int ds_event(Lane<T>& L, const C& c, const ElecRng& g
 
 // ---------------------------------------------------------------------------
 // continuous event (MC/tools/scattering.py:753-883 in the order of
-// MC/tools/singleScatter.py:210-239, with the Bethe law the mode names)
+// MC/tools/singleScatter.py:210-239, with the Bethe law the mode names).  With
+// s2_out the direction update is left to the caller.
 // ---------------------------------------------------------------------------
 template <class T, bool REC, class C>
 __device__ __forceinline__ int cont_event_r(Lane<T>& L, const C& c, const uint4 r, EventOut<T>* ev,
-                                            const EventPre<T>* pre = nullptr) {
+                                            const EventPre<T>* pre = nullptr, T* s2_out = nullptr) {
     const T E = L.E;
     const T sR = sig_ruth<T>(c, E);
     const T s = -(pre ? pre->ln_y : Ops<T>::ln_step_word(r.y)) * Ops<T>::div((T)1, sR);
@@ -1012,7 +1013,9 @@ __device__ __forceinline__ int cont_event_r(Lane<T>& L, const C& c, const uint4 
     }
     const bool left = L.outcome != MCD_OUT_NONE;
     if (!left || (c.bits & MCD_Q_CROSSING_STEP)) lane_lose(L, c, dE);
-    if (L.outcome == MCD_OUT_NONE) {
+    if (s2_out) {
+        *s2_out = s2;
+    } else if (L.outcome == MCD_OUT_NONE) {
         if (pre) lane_rotate_cs(L, s2, pre->cph, pre->sph);
         else lane_rotate(L, c, s2, r.w);
     }

@@ -157,7 +157,8 @@ struct GroupTurn {
 // a warp instruction and a small run's warps share it, so 25 of the event's 77
 // FP64 instructions (35 of the update become 10) are time, and the shuffles
 // that come instead are not: 1000 Si 10 keV electrons 2.51 -> 2.13
-// ms, 700 Au 20 keV 9.8 -> 8.0, 3000 Si 3.7 -> 3.2 (with their host calls).
+// ms, 700 Au 20 keV 9.8 -> 8.0, 3000 Si 3.7 -> 3.2, 1000 Cu in the continuous
+// model 4.08 -> 3.82 (with their host calls).
 template <int G>
 __device__ __forceinline__ void group_turn(Lane<double>& L, const GroupTurn<double>& turn, double cph, double sph,
                                            const GroupLanes<G>& g) {

@@ -70,20 +70,22 @@ __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst
         const EventPre<T> next = pre[((step + 1) / G) & 1][g.h0 + (int)((step + 1) & (G - 1))];
         EventOut<T> ev;
         int ch = kGroupNone;
+        GroupTurn<T> turn{(T)0, false};
         if (MODE == MCD_MODE_DS) {
-            GroupTurn<T> turn{(T)0, false};
             ch = group_event<T, REC, G>(L, sig, c, cur, active, w.w, g, zmax, use_tab, &ev, &turn);
-            if constexpr (sizeof(T) == 8) {
-                if (G < 32) __syncwarp();
-                group_turn<G>(L, turn, cur.cph, cur.sph, g);
-            }
         } else if (active) {
             if (step >= w.w) {
                 lane_long(L);
             } else {
                 L.step = step + 1;
-                ch = cont_event_r<T, REC>(L, c, make_uint4(0u, 0u, cur.rz, cur.rw), &ev, &cur);
+                ch = cont_event_r<T, REC>(L, c, make_uint4(0u, 0u, cur.rz, cur.rw), &ev, &cur,
+                                          sizeof(T) == 8 ? &turn.s2 : nullptr);
+                turn.due = L.outcome == MCD_OUT_NONE;
             }
+        }
+        if constexpr (sizeof(T) == 8) {
+            if (G < 32) __syncwarp();
+            group_turn<G>(L, turn, cur.cph, cur.sph, g);
         }
         if (REC && g.t == 0 && ch != kGroupNone) st |= ring_append(ring, (uint32_t)i, L.step, ev);
         if (ch != kGroupPlain && active) {

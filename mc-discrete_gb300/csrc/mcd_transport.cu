@@ -545,15 +545,15 @@ static int dispatch_plain(const SimConst<T>& c, int block, mcd_tally* tally, con
 //                        9000: 25.4 / 29.8, 11000 35.3 / 29.0; Au 14000: 63 / 116
 //                        (the plain kernel evaluates a cross section per
 //                        shell in every event)
-//   FP64 continuous      300: 3.69 / 3.81 with 32 / 8;  1500: 3.99 / 4.55 with 8
-//                        / 0;  2500: 4.72 / 4.54
+//   FP64 continuous (Cu) 450: 3.72 / 3.82 with 32 / 8, 700: 4.21 / 3.85;  2500:
+//                        4.53 / 4.83 with 8 / 0, 4000: 5.93 / 5.08
 static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) {
     const int64_t e = s.num_el / sms;   // electrons per SM
     if (s.precision == MCD_FP32) {
         if (s.mode != MCD_MODE_DS) return e < 12 ? 32 : e < 34 ? 8 : 0;
         return e < 20 ? 32 : e < 33 ? 16 : e < 58 ? 8 : 0;
     }
-    if (s.mode != MCD_MODE_DS) return e < 3 ? 32 : e < 10 ? 8 : 0;
+    if (s.mode != MCD_MODE_DS) return e < 3 ? 32 : e < 18 ? 8 : 0;
     const int most = s.sigma_table ? 47 : 16 * (m.n_shells > 3 ? m.n_shells : 3);
     return e < 7 ? 32 : e < 12 ? 16 : e < most ? 8 : 0;
 }
