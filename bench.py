@@ -47,22 +47,21 @@ MUFU_PER_EVENT = {k: 17 + 4 * n for k, n in N_SHELLS.items()}     # Si 29, Au 49
 # proportion to num_el, so that its mix of trajectory lengths is the workload's
 CPU_SAMPLE_ELECTRONS = 40000
 # DRAM bytes (read + write) of one batched launch of the 64-simulation step,
-# from an ncu capture of that launch (tables and workspace read about once;
-# the figure does not grow with the electrons)
-BATCHED_DRAM_BYTES = 55.48e6 + 0.47e6
-# warp instructions issued per event by the batched kernel on this workload
-# in its tuned shape (two blocks of 576 per SM, 56 registers), from an ncu
-# capture of a quarter-size launch (2.0065e10 instructions for 1.3855e9
-# events); the issue peak is one warp instruction per scheduler per cycle,
-# 4 schedulers per SM
-WARP_INST_PER_EVENT = 14.48
-# the same capture's unit fractions (of peak sustained): issue-active cycles,
-# threads per warp instruction / 32, the L1/TEX unit, its shared-memory
-# wavefronts, and L2
-BATCHED_NCU = {"issue_active": 0.770, "warp_execution_efficiency": 0.714, "l1tex_throughput": 0.747,
-               "shared_wavefronts": 0.301, "l2_throughput": 0.029,
-               "capture": "ncu --set full of k_batched_lr (2 x 576, 56 registers) on a quarter of the workload "
-                          "(1.3855e9 events)"}
+# (the persistent kernel and the run-down kernel after it) from an ncu capture
+# of a smaller launch of the same simulations: tables and workspace read about
+# once, and the run-down kernel's list; the figure does not grow with the
+# electrons
+BATCHED_DRAM_BYTES = 54.46e6 + 2.39e6 + 19.41e6
+# warp instructions issued per event by both kernels on this workload in its
+# tuned shape (two blocks of 576 per SM, 56 registers), from that capture
+# (2.167e10 and 6.99e8 instructions for 1.7539e9 events); the issue peak is one
+# warp instruction per scheduler per cycle, 4 schedulers per SM
+WARP_INST_PER_EVENT = 12.75
+# the same capture's fractions of the persistent kernel: issue-active cycles,
+# threads per warp instruction / 32, the L1/TEX unit
+BATCHED_NCU = {"issue_active": 0.757, "warp_execution_efficiency": 0.775, "l1tex_throughput": 0.84,
+               "capture": "ncu counters of k_batched_lr (2 x 576, 56 registers) on the 64 simulations with "
+                          "10^U[2.5, 5.5] electrons (1.7539e9 events)"}
 
 
 def workload(scale=1.0):
@@ -282,9 +281,8 @@ def cfg1_bench(args, dev):
             "gpu_inline_ms": ms_inline, "gpu_fp32_ms": ms32,
             "longest_electron_events": int(g.electrons["n_events"].max()),
             "note": "the launch lasts as long as its longest trajectory, a chain of dependent instructions "
-                    "(FP64 ones the longest); the automatic size runs two electrons per warp (at most one "
-                    "warp per scheduler), each on a half-warp whose lanes compute the next 16 events' "
-                    "trajectory-independent values (Philox block, step logarithm, azimuth, uniforms)",
+                    "(FP64 ones the longest); the automatic size runs several lanes per electron, which look "
+                    "ahead in the random stream and share the cross sections and the direction update",
             "cpu_1core_s": cpu[1], "cpu_all_cores_s": cpu[os.cpu_count() or 1], "cpu_cores": os.cpu_count() or 1,
             "cpu_timing": "best of 3 on all cores, one run on 1 core",
             "eta_gpu_fp64": g.tally["bks"] / n, "eta_oracle": float(np.mean(c["outcome"] == 1)),
@@ -402,7 +400,7 @@ def adjoint_bench(args, dev):
             "bwd_over_fwd": tb / tf, "loss": L, "dL_dJscale": dJ, "dL_dnscale": dn,
             "fd_frozen_dL_dJscale": fd, "fd_frozen_rel_err": abs(dJ - fd) / abs(fd) if fd else None,
             "fd_crn": crn, "fd_crn_rel_err": crn["rel_err"],
-            "fd_step": d, "max_depth": depth, "gpu_launches": 2 * args.steps + depth["gpu_launches"] + 3}
+            "fd_step": d, "max_depth": depth, "gpu_launches": 3 * args.steps + depth["gpu_launches"] + 3}
 
 
 def adjoint_depth_bench(args, dev, p, n):
@@ -454,7 +452,7 @@ def adjoint_depth_bench(args, dev, p, n):
             "dL_dJscale": dJ, "dL_dnscale": dn, "fd_frozen_rel_err_J": abs(dJ - fdJ) / abs(fdJ) if fdJ else None,
             "fd_frozen_rel_err_n": abs(dn - fdn) / abs(fdn) if fdn else None, "fd_step": d,
             "fp64_electrons": n64, "fp64_fd_frozen_rel_err_J": abs(dJ64 - fdJ64) / abs(fdJ64) if fdJ64 else None,
-            "gpu_launches": 2 * args.steps + 6}
+            "gpu_launches": 3 * args.steps + 6}
 
 
 TABLES_WORKLOAD = ("the sampled-loss table pairs (Moller, outermost-shell Gryzinski) of the 16 (material, E0) "
@@ -569,7 +567,7 @@ def cont_bench(args, dev):
             "cpu_baseline": None if args.no_cpu else oracle_eta_check(
                 args, t["bks"] / n, n, _oracle_material("Cu"), 20000.0, 1000.0, 70.0, min(n, 20000),
                 mode="cont", bethe="JL", max_scatt=10 ** 6),
-            "gpu_launches": 2 * args.steps}
+            "gpu_launches": 3 * args.steps}
 
 
 def _oracle_material(sp):
@@ -706,7 +704,7 @@ def stream_bench(args, dev):
             "drain_GB_per_s": drain, "d2h_link_GB_per_s": link, "drain_frac_of_link": drain / link,
             "record_bytes": es.rec_bytes,
             "ring_GB": es.cap * es.rec_bytes / 1e9, "eta": eta, "cpu_baseline": cpu,
-            "reruns": st["reruns"], "gpu_launches": len(es.batches)}
+            "reruns": st["reruns"], "gpu_launches": 2 * len(es.batches)}
 
 
 def run_mcd(args):
@@ -883,7 +881,7 @@ def run_mcd(args):
     top, name = (mufu_, "mufu-issue") if mufu_["frac"] >= fp32["frac"] else (fp32, "fp32-issue")
     roofline = {"bound": name, "achieved": top["achieved"], "peak": top["peak"], "unit": top["unit"],
                 "frac": top["frac"], "traffic": BATCHED_DRAM_BYTES if args.scale == 1.0 else None,
-                "traffic_note": "DRAM bytes per launch from an ncu capture of the full step",
+                "traffic_note": "DRAM bytes per launch from an ncu capture of a smaller step",
                 "fp32": fp32, "mufu": mufu_,
                 "issue": {"achieved": value * WARP_INST_PER_EVENT / 1e9 / ws,
                           "peak": sms * 4 * fmax / 1e9, "unit": "G warp instructions/s",
@@ -955,7 +953,7 @@ def run_mcd(args):
         "cfg1": c1,
         "detector": det,
         "tables": tabs,
-        "gpu_launches": K,
+        "gpu_launches": 2 * K,   # the persistent kernel and the run-down kernel after it
         "status": status,
     }
     print(json.dumps(line), flush=True)
