@@ -143,11 +143,31 @@ struct GroupLanes {
         : t(lane & (G - 1)), h0(lane & ~(G - 1)), gmask(ones << (lane & ~(G - 1))) {}
 };
 
-// The direction update that an FP64 event leaves to group_turn
-template <class T>
+// (FP64) A Rutherford event's sin^2(theta/2) and what the direction update takes
+// of it: cos(theta) and sin(theta) cos(phi), sin(theta) sin(phi).  They depend on
+// the energy and on the event's random values alone, so each lane computes them
+// for its event of those ahead, and again when the energy has changed: 23 of the
+// event's 48 FP64 instructions, which most events then need not issue.  1000 Si 10
+// keV electrons 2.30 -> 2.03 ms, 1000 Au 20 keV 7.75 -> 5.50 (with their host
+// calls).  In FP32, where the instructions are cheap and the shared memory's
+// latency is not, the same lost 3 to 6%.
+struct GroupAngle {
+    double s2, cth, a, b;
+};
+__device__ __forceinline__ GroupAngle group_deflect(double s2, double cph, double sph) {
+    const double sth = 2.0 * Ops<double>::sqrt_(s2 * (1.0 - s2));   // the operations of lane_rotate_cs
+    return GroupAngle{s2, 1.0 - 2.0 * s2, sth * cph, sth * sph};
+}
+template <class C>
+__device__ __forceinline__ GroupAngle group_angle(const C& c, double E, const EventPre<double>& p) {
+    return group_deflect(ruth_s2<double>(c, E, p.a0u, p.uzc), p.cph, p.sph);
+}
+
+// What an FP64 event takes of the angles computed ahead and leaves to group_turn
 struct GroupTurn {
-    T s2;
-    bool due;
+    GroupAngle t;    // of the event as a Rutherford one; then the event's
+    bool due;        // the direction is to be updated
+    bool changed;    // the energy has changed, and goes on
 };
 
 // lane_rotate_cs by the lanes of a group, called by the whole warp: lane q of
@@ -160,10 +180,9 @@ struct GroupTurn {
 // ms, 700 Au 20 keV 9.8 -> 8.0, 3000 Si 3.7 -> 3.2, 1000 Cu in the continuous
 // model 4.08 -> 3.82 (with their host calls).
 template <int G>
-__device__ __forceinline__ void group_turn(Lane<double>& L, const GroupTurn<double>& turn, double cph, double sph,
+__device__ __forceinline__ void group_turn(Lane<double>& L, const GroupTurn& turn, double cph, double sph,
                                            const GroupLanes<G>& g) {
-    const double s2 = turn.s2, sth = 2.0 * Ops<double>::sqrt_(s2 * (1.0 - s2)), cth = 1.0 - 2.0 * s2;
-    const double a = sth * cph, b = sth * sph;
+    const double cth = turn.t.cth, a = turn.t.a, b = turn.t.b;
     const int q = g.t % 6, i = q % 3;
     const bool axis = q >= 3;
     auto pick = [](int k, double x, double y, double z) { return k == 0 ? x : k == 1 ? y : z; };
@@ -190,15 +209,15 @@ __device__ __forceinline__ void group_turn(Lane<double>& L, const GroupTurn<doub
 constexpr int kGroupNone = -1;    // the group took no event (no electron, or at the event limit)
 constexpr int kGroupPlain = -2;   // a Rutherford event that stays in the sample
 
-// One DS event of every group of a warp, but in FP64 for its direction update
-// (called by all its lanes; active: the
-// group has an electron; cur: its event's values computed ahead).  Returns the
-// channel code, kGroupNone or kGroupPlain; the step counter has advanced
-// unless it is kGroupNone.
+// One DS event of every group of a warp, but in FP64 for its direction update,
+// which is left in *turn (called by all its lanes; active: the group has an
+// electron; cur: its event's values computed ahead).  Returns the channel code,
+// kGroupNone or kGroupPlain; the step counter has advanced unless it is
+// kGroupNone.
 template <class T, bool REC, int G, class C>
 __device__ __forceinline__ int group_event(Lane<T>& L, GroupSig<T, G>& sig, const C& c, const EventPre<T>& cur,
                                            bool active, uint32_t limit, const GroupLanes<G>& g, T zmax, bool use_tab,
-                                           EventOut<T>* ev, GroupTurn<T>* turn = nullptr) {
+                                           EventOut<T>* ev, GroupTurn* turn = nullptr) {
     // the columns passed: 0 Rutherford, 1 Moller, 2.. Gryz, K-1 Quinn
     const T level = cur.ux * sig.all;
     unsigned below = 0;
@@ -214,7 +233,9 @@ __device__ __forceinline__ int group_event(Lane<T>& L, GroupSig<T, G>& sig, cons
     if (!active) return kGroupNone;
     // what a Rutherford event does; the others replace it
     const T E = L.E;
-    T W = (T)0, s2 = ruth_s2<T>(c, E, cur.a0u, cur.uzc), path = -cur.ln_y * sig.mfp;
+    T W = (T)0, s2, path = -cur.ln_y * sig.mfp;
+    if constexpr (sizeof(T) == 8) s2 = turn->t.s2;
+    else s2 = ruth_s2<T>(c, E, cur.a0u, cur.uzc);
     int ch = MCD_CH_RUTH;
     if (sizeof(T) == 4) {
         // a Rutherford event that stays in the sample changes nothing but the
@@ -260,13 +281,16 @@ __device__ __forceinline__ int group_event(Lane<T>& L, GroupSig<T, G>& sig, cons
             s2 = collide(L, c, E, W);
         }
         const T after = E - W;
-        if (loss && after > c.Emin) group_sig<T, G>(c, after, use_tab, g.t, g.h0, g.gmask, sig);
+        if (loss && after > c.Emin) {
+            group_sig<T, G>(c, after, use_tab, g.t, g.h0, g.gmask, sig);
+            if constexpr (sizeof(T) == 8) turn->changed = true;
+        }
     }
     if (REC) event_out<T>(*ev, L, E, W, path, s2, cur.rw, ch);
     lane_move(L, c, path, ch == MCD_CH_DIFF);
     if (loss && (L.outcome == MCD_OUT_NONE || (c.bits & MCD_Q_CROSSING_STEP))) lane_lose(L, c, W);
     if constexpr (sizeof(T) == 8) {
-        turn->s2 = s2;
+        if (ch != MCD_CH_RUTH) turn->t = group_deflect(s2, cur.cph, cur.sph);
         turn->due = L.outcome == MCD_OUT_NONE;
     } else if (L.outcome == MCD_OUT_NONE) {
         lane_rotate_cs(L, s2, cur.cph, cur.sph);

@@ -15,7 +15,10 @@
 //    column of the table (or one shell's expression) per lane, and an event's
 //    channel is one comparison per lane and a vote;
 //  - a W table's interval is found by comparing the guide's range of entries
-//    with the draw, one entry per lane.
+//    with the draw, one entry per lane;
+//  - in FP64, whose pipe the warps of an SM share, the polar angles of the events
+//    ahead are computed one per lane, again where the energy changes, and the
+//    direction update's components one per lane (mcd_group.cuh).
 // The trajectories are the plain kernel's, bit for bit.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -33,12 +36,17 @@ constexpr int lanes_blocks(int group) {
     return sizeof(T) == 4 ? (group == 8 ? 20 : 16) : (group == 8 ? 16 : 1);
 }
 
+// where the continuous FP64 event leaves its sin^2(theta/2)
+__device__ __forceinline__ double* turn_s2(GroupTurn* t, double) { return &t->t.s2; }
+__device__ __forceinline__ float* turn_s2(GroupTurn*, float) { return nullptr; }
+
 template <class T, int MODE, bool REC, int G>
 __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst<T> cp, mcd_tally* tally, const ElOut eo,
                                               const mcd_event_ring ring, uint32_t* status) {
     __shared__ BlockTally bt;
     __shared__ SimConst<T> full;
     __shared__ EventPre<T> pre[2][32];
+    __shared__ GroupAngle angles[32];   // (FP64 DS) of the block of events under way
     if (threadIdx.x == 0) full = cp;
     bt_zero(&bt, 1);
     __syncwarp();
@@ -62,15 +70,30 @@ __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst
     pre[0][lane] = event_pre<T>(c, philox_event(rng, (uint32_t)g.t, w), ang);
     __syncwarp();
     EventPre<T> cur = pre[0][g.h0];
+    constexpr bool kAngles = sizeof(T) == 8 && MODE == MCD_MODE_DS;
+    GroupTurn turn{};
+    turn.changed = true;   // angles[] are of another block or energy
     while (G == 32 ? active : __any_sync(0xffffffffu, active)) {
         if ((step & (G - 1)) == 0) {   // the block of events after this one
             pre[(step / G + 1) & 1][lane] = event_pre<T>(c, philox_event(rng, step + G + (uint32_t)g.t, w), ang);
             __syncwarp();
+            turn.changed = true;
+        }
+        GroupAngle angle_next{};
+        if constexpr (kAngles) {
+            if (G == 32 ? turn.changed : __any_sync(0xffffffffu, turn.changed)) {
+                __syncwarp();
+                angles[lane] = group_angle(c, L.E, pre[(step / G) & 1][lane]);
+                __syncwarp();
+                turn.t = angles[g.h0 + (int)(step & (G - 1))];
+                turn.changed = false;
+            }
+            angle_next = angles[g.h0 + (int)((step + 1) & (G - 1))];
         }
         const EventPre<T> next = pre[((step + 1) / G) & 1][g.h0 + (int)((step + 1) & (G - 1))];
         EventOut<T> ev;
         int ch = kGroupNone;
-        GroupTurn<T> turn{(T)0, false};
+        turn.due = false;
         if (MODE == MCD_MODE_DS) {
             ch = group_event<T, REC, G>(L, sig, c, cur, active, w.w, g, zmax, use_tab, &ev, &turn);
         } else if (active) {
@@ -79,7 +102,8 @@ __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst
             } else {
                 L.step = step + 1;
                 ch = cont_event_r<T, REC>(L, c, make_uint4(0u, 0u, cur.rz, cur.rw), &ev, &cur,
-                                          sizeof(T) == 8 ? &turn.s2 : nullptr);
+                                          turn_s2(&turn, (T)0));
+                if (sizeof(T) == 8) turn.t = group_deflect(turn.t.s2, (double)cur.cph, (double)cur.sph);
                 turn.due = L.outcome == MCD_OUT_NONE;
             }
         }
@@ -96,6 +120,7 @@ __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst
             }
         }
         cur = next;
+        if (kAngles) turn.t = angle_next;
         ++step;
     }
     or_status(status, st);

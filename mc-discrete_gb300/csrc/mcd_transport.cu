@@ -536,11 +536,12 @@ static int dispatch_plain(const SimConst<T>& c, int block, mcd_tally* tally, con
 //   0.85, 4500 0.95 / 1.08, 7500 1.21 / 1.23, 10000 1.36 / 1.32)
 //   FP32 continuous      1500: 0.21 / 0.23 with 32 / 8;  2500: 0.28 / 0.24;
 //                        4500: 0.25 / 0.27 with 8 / 0;  6500: 0.28 / 0.28
-//   FP64 DS (with their host calls; Si, table)  1000: 2.35 / 2.33 with 32 / 16,
-//                        1300: 2.57 / 2.36;  1800: 2.56 / 2.70 with 16 / 8, 2500:
-//                        4.17 / 3.15;  6500: 4.88 / 5.35 with 8 / 0, 7500: 5.56 / 5.34
-//   (Au: 1000 7.98 / 8.69 with 32 / 16, 1300 9.24 / 8.90, 1800 9.21 / 9.76 with
-//   16 / 8, 2500 10.5 / 10.1, 9000 21.2 / 26.3 with 8 / 0)
+//   FP64 DS (with their host calls; Si, table)  1200: 2.15 / 2.31 with 32 / 16,
+//                        1400: 2.63 / 2.37;  2100: 2.60 / 2.82 with 16 / 8, 2500:
+//                        3.76 / 3.10 (up to two warps per scheduler, both);
+//                        6500: 4.9 / 5.35 with 8 / 0, 7500: 5.6 / 5.34
+//   (Au: 1200 6.00 / 6.20 with 32 / 16, 1400 6.01 / 6.25, 2100 6.64 / 7.80 with
+//   16 / 8, 2500 6.99 / 8.14, 9000 21.2 / 26.3 with 8 / 0)
 //   without a table      Si 7000: 15.7 / 16.5 with 8 / 0, 9000 19.9 / 16.7; Cu
 //                        9000: 25.4 / 29.8, 11000 35.3 / 29.0; Au 14000: 63 / 116
 //                        (the plain kernel evaluates a cross section per
@@ -555,7 +556,7 @@ static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) 
     }
     if (s.mode != MCD_MODE_DS) return e < 3 ? 32 : e < 18 ? 8 : 0;
     const int most = s.sigma_table ? 47 : 16 * (m.n_shells > 3 ? m.n_shells : 3);
-    return e < 7 ? 32 : e < 12 ? 16 : e < most ? 8 : 0;
+    return e < 8 ? 32 : e < 16 ? 16 : e < most ? 8 : 0;
 }
 
 // Does an automatic run of a thread per electron take one resident block per

@@ -22,7 +22,7 @@ RUNS = {
     "cont_ex": dict(input_par("Al", 5000.0, 1000.0, 0.0, mode="cont", bethe="explicit"), maxScatt=150),
 }
 SMS = 152
-# electrons per SM: below 3, 7, 12, 18, 20, 33, 34, 47 and 58 the group width changes
+# electrons per SM: below 3, 8, 16, 18, 20, 33, 34, 47 and 58 the group width changes
 SIZES = [1, 2, 3, 31, 2 * SMS + 1, 4 * SMS, 9 * SMS + 5, 11 * SMS, 25 * SMS + 3, 40 * SMS + 7]
 
 
@@ -49,8 +49,8 @@ def test_rows_equal_plain(name, n, tabulated, precision):
     same(engine.run(p, **kw), engine.run(p, block_size=64, **kw))
 
 
-@pytest.mark.parametrize("n", [7 * SMS - 1, 7 * SMS, 12 * SMS - 1, 12 * SMS, 18 * SMS - 1, 18 * SMS, 47 * SMS - 1, 47 * SMS])
-@pytest.mark.parametrize("name", ["si", "film", "limit", "cont"])
+@pytest.mark.parametrize("n", [8 * SMS - 1, 8 * SMS, 16 * SMS - 1, 16 * SMS, 18 * SMS - 1, 18 * SMS, 47 * SMS - 1, 47 * SMS])
+@pytest.mark.parametrize("name", ["si", "au", "film", "limit", "cont"])
 def test_fp64_rows_equal_plain_at_the_widths(name, n):
     kw = dict(num_el=n, seed=n, precision="fp64", tabulated=True, tally_channels=True)
     same(engine.run(RUNS[name], **kw), engine.run(RUNS[name], block_size=64, **kw))
