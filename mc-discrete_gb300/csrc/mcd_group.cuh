@@ -176,9 +176,9 @@ struct GroupTurn {
 // every lane of the group receives all six.  The FP64 pipe takes 16 cycles for
 // a warp instruction and a small run's warps share it, so 25 of the event's 77
 // FP64 instructions (35 of the update become 10) are time, and the shuffles
-// that come instead are not: 1000 Si 10 keV electrons 2.51 -> 2.13
-// ms, 700 Au 20 keV 9.8 -> 8.0, 3000 Si 3.7 -> 3.2, 1000 Cu in the continuous
-// model 4.08 -> 3.82 (with their host calls).
+// that come instead are not: 1000 Si 10 keV electrons 2.72 -> 2.37 ms, 700 Au 20
+// keV 9.76 -> 7.98, 3000 Si 3.74 -> 3.22, 1000 Cu in the continuous model 4.08 ->
+// 3.82 (with their host calls).
 template <int G>
 __device__ __forceinline__ void group_turn(Lane<double>& L, const GroupTurn& turn, double cph, double sph,
                                            const GroupLanes<G>& g) {
