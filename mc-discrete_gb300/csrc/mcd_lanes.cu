@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst
     turn.changed = true;   // angles[] are of another block or energy
     while (G == 32 ? active : __any_sync(0xffffffffu, active)) {
         if ((step & (G - 1)) == 0) {   // the block of events after this one
+            __syncwarp();   // it takes the place of one whose values other lanes may still be reading
             pre[(step / G + 1) & 1][lane] = event_pre<T>(c, philox_event(rng, step + G + (uint32_t)g.t, w), ang);
             __syncwarp();
             turn.changed = true;
