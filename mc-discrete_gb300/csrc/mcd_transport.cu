@@ -757,9 +757,13 @@ static int read_tune(const mcd_tune* tune, int* block, int* per_sm, int* refill)
     return MCD_OK;
 }
 
+// Dynamic shared memory beyond what a block has without asking for more: 48 KB
+// less the kernel's static arrays (the run-down kernel has some 500 bytes).
 template <class K>
 static int set_smem(K kern, size_t smem) {
-    if (smem <= 48 * 1024) return MCD_OK;
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, kern) != cudaSuccess) return MCD_ECUDA;
+    if (smem + a.sharedSizeBytes <= 48 * 1024) return MCD_OK;
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess
                ? MCD_OK
                : MCD_ECUDA;
