@@ -1157,6 +1157,25 @@ __device__ __forceinline__ uint32_t ring_append(const mcd_event_ring& ring, uint
     return takes ? 0u : MCD_FLAG_RING_INDEX;
 }
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory.  What a block
+// has without asking for more is 48 KB less the kernel's static arrays (the
+// run-down kernel has some 500 bytes); a kernel that needs more is allowed all
+// that the device has, always the same value, so that a launch of another size
+// by another thread never takes back what this one has asked for.
+inline int allow_smem(const void* kern, size_t bytes) {
+    cudaFuncAttributes a;
+    if (cudaFuncGetAttributes(&a, kern) != cudaSuccess) return MCD_ECUDA;
+    if (bytes + a.sharedSizeBytes <= 48 * 1024) return MCD_OK;
+    int dev = 0, most = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return MCD_ECUDA;
+    const size_t all = (size_t)most - a.sharedSizeBytes;
+    if (bytes > all) return MCD_ECUDA;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)all) == cudaSuccess ? MCD_OK
+                                                                                                           : MCD_ECUDA;
+}
+
 }  // namespace mcd
 
 #endif  // MCD_DEVICE_CUH

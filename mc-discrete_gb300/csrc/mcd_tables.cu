@@ -375,9 +375,7 @@ extern "C" int mcd_build_table(int kind, const mcd_material* mat, int shell, int
     const bool smem = nW - 1 <= kFillCols;
     const size_t bytes = smem ? fill_smem(w, nW) : 0;
     auto kern = smem ? k_fill<true> : k_fill<false>;
-    if (bytes > 48 * 1024 &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-        return MCD_ECUDA;
+    if (allow_smem((const void*)kern, bytes) != MCD_OK) return MCD_ECUDA;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, 32 * w, bytes) != cudaSuccess) return MCD_ECUDA;
     if (fit < 1) return MCD_ETOOBIG;
     const long long rows = ((long long)nE + w - 1) / w, cap = (long long)sms * fit;

@@ -757,18 +757,6 @@ static int read_tune(const mcd_tune* tune, int* block, int* per_sm, int* refill)
     return MCD_OK;
 }
 
-// Dynamic shared memory beyond what a block has without asking for more: 48 KB
-// less the kernel's static arrays (the run-down kernel has some 500 bytes).
-template <class K>
-static int set_smem(K kern, size_t smem) {
-    cudaFuncAttributes a;
-    if (cudaFuncGetAttributes(&a, kern) != cudaSuccess) return MCD_ECUDA;
-    if (smem + a.sharedSizeBytes <= 48 * 1024) return MCD_OK;
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess
-               ? MCD_OK
-               : MCD_ECUDA;
-}
-
 // The persistent launch and, where the list can hold an electron per lane and
 // the run-down kernel's block fits, that kernel after it.
 template <bool REC>
@@ -785,14 +773,14 @@ static int launch_batched(void* workspace, int nsims, mcd_tally* tallies, const 
     const size_t smem = batch_smem(nsims), smem2 = batch_drain_off(nsims) + drain_smem(kDrainThreads);
     auto kern = k_batched<REC>;
     if constexpr (!REC) kern = lowreg ? k_batched_lr<false> : k_batched<false>;
-    if (set_smem(kern, smem) != MCD_OK) return MCD_ECUDA;
+    if (allow_smem((const void*)kern, smem) != MCD_OK) return MCD_ECUDA;
     int fit = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, block, smem) != cudaSuccess) return MCD_ECUDA;
     if (fit < 1) return MCD_ETOOBIG;
     if (per_sm <= 0 || per_sm > fit) per_sm = fit;
     if ((long long)sms * per_sm * block <= kLiveSeats && smem2 + 1024 <= (size_t)most) flags |= kRunList;
     auto down = nsims == 1 ? k_rundown<REC, true> : k_rundown<REC, false>;
-    if ((flags & kRunList) && set_smem(down, smem2) != MCD_OK) return MCD_ECUDA;
+    if ((flags & kRunList) && allow_smem((const void*)down, smem2) != MCD_OK) return MCD_ECUDA;
     // reset the queue and the list (the first two words of the workspace)
     if (cudaMemsetAsync(workspace, 0, 2 * sizeof(unsigned long long), st) != cudaSuccess) return MCD_ECUDA;
     uint8_t* ws = static_cast<uint8_t*>(workspace);
@@ -959,9 +947,7 @@ extern "C" int mcd_run_batched_noalloc(const mcd_sim* sims, int32_t nsims, const
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return MCD_ECUDA;
     const size_t smem = batch_smem(nsims);
     auto kern = lowreg ? k_batched_lr<false> : k_batched<false>;
-    if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return MCD_ECUDA;
+    if (allow_smem((const void*)kern, smem) != MCD_OK) return MCD_ECUDA;
     int fit = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, block, smem) != cudaSuccess) return MCD_ECUDA;
     if (fit < 1) return MCD_ETOOBIG;
