@@ -183,7 +183,8 @@ __device__ __forceinline__ bool run_cont(const C& c) {
     return Sims::MODE == MCD_MODE_CONT || (Sims::MODE == kMixed && (c.bits & kBitCont));
 }
 
-// Runs the electrons of a warp's groups for up to `events` events each.
+// Runs the electrons of a warp's groups, which have had an event (so that their
+// energy is above Emin), for up to `events` events each.
 template <bool REC, bool CHAN, int G, class Sims>
 __device__ __forceinline__ uint32_t group_run(const Sims& s, int sim, Lane<float>& L, const ElecRng& rng, bool& have,
                                               int events, EventPre<float>* buf, const mcd_event_ring& ring,
@@ -221,7 +222,7 @@ __device__ __forceinline__ uint32_t group_run(const Sims& s, int sim, Lane<float
         }
         int ch = kGroupNone;
         if (Sims::MODE != MCD_MODE_CONT)
-            ch = group_event<float, REC, G>(L, sig, c, cur, have && !cont, w.w, g, zmax, use_tab, &ev);
+            ch = group_event<float, REC, G>(L, sig, c, cur, have && !cont, w.w, w.w, g, zmax, use_tab, &ev);
         if (have && cont) {
             if (L.step >= w.w) {
                 lane_long(L);

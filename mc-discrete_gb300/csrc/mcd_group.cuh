@@ -213,11 +213,13 @@ constexpr int kGroupPlain = -2;   // a Rutherford event that stays in the sample
 // which is left in *turn (called by all its lanes; active: the group has an
 // electron; cur: its event's values computed ahead).  Returns the channel code,
 // kGroupNone or kGroupPlain; the step counter has advanced unless it is
-// kGroupNone.
+// kGroupNone.  plain: the events below which an event that loses no energy may
+// go on without the test E > Emin: the limit, or 0 for a beam that is not above
+// Emin (group_plain), whose electrons end with their first event.
 template <class T, bool REC, int G, class C>
 __device__ __forceinline__ int group_event(Lane<T>& L, GroupSig<T, G>& sig, const C& c, const EventPre<T>& cur,
-                                           bool active, uint32_t limit, const GroupLanes<G>& g, T zmax, bool use_tab,
-                                           EventOut<T>* ev, GroupTurn* turn = nullptr) {
+                                           bool active, uint32_t limit, uint32_t plain, const GroupLanes<G>& g, T zmax,
+                                           bool use_tab, EventOut<T>* ev, GroupTurn* turn = nullptr) {
     // the columns passed: 0 Rutherford, 1 Moller, 2.. Gryz, K-1 Quinn
     const T level = cur.ux * sig.all;
     unsigned below = 0;
@@ -244,7 +246,7 @@ __device__ __forceinline__ int group_event(Lane<T>& L, GroupSig<T, G>& sig, cons
         // the groups of a warp would each issue their own rotation, it lost
         // (1000 Si electrons 2.42 -> 2.96 ms)
         const T nz = L.z + path * L.dz;
-        if (j == 0 && !dif && !(nz <= (T)0) && !(nz >= zmax) && L.step < limit) {
+        if (j == 0 && !dif && !(nz <= (T)0) && !(nz >= zmax) && L.step < plain) {
             if (REC) event_out<T>(*ev, L, E, W, path, s2, cur.rw, ch);
             L.step += 1;
             lane_move(L, c, path);
@@ -288,7 +290,7 @@ __device__ __forceinline__ int group_event(Lane<T>& L, GroupSig<T, G>& sig, cons
     }
     if (REC) event_out<T>(*ev, L, E, W, path, s2, cur.rw, ch);
     lane_move(L, c, path, ch == MCD_CH_DIFF);
-    if (loss && (L.outcome == MCD_OUT_NONE || (c.bits & MCD_Q_CROSSING_STEP))) lane_lose(L, c, W);
+    if ((loss || plain == 0) && (L.outcome == MCD_OUT_NONE || (c.bits & MCD_Q_CROSSING_STEP))) lane_lose(L, c, W);
     if constexpr (sizeof(T) == 8) {
         if (ch != MCD_CH_RUTH) turn->t = group_deflect(s2, cur.cph, cur.sph);
         turn->due = L.outcome == MCD_OUT_NONE;
@@ -296,6 +298,12 @@ __device__ __forceinline__ int group_event(Lane<T>& L, GroupSig<T, G>& sig, cons
         lane_rotate_cs(L, s2, cur.cph, cur.sph);
     }
     return ch;
+}
+
+// group_event's `plain`: FP32 can round E0 to Emin (E0 > Emin is checked in FP64)
+template <class T>
+__device__ __forceinline__ uint32_t group_plain(const SimConst<T>& c) {
+    return sizeof(T) == 8 || c.E0 > c.Emin ? c.max_scatt : 0u;
 }
 
 // the bottom face as group_event tests it

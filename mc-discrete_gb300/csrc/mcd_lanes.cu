@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst
     const uint4 w = event_words(c);   // sim id and Philox key words, event limit
     const bool chan = (full.tally_flags & MCD_TALLY_CHANNELS) != 0;
     const T zmax = group_zmax<T>(c);
+    const uint32_t plain = group_plain(full);
     const bool use_tab = c.sig != nullptr;
     const T ang = MODE == MCD_MODE_DS ? c.a0 : (T)1;
     Lane<T> L;
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst
         int ch = kGroupNone;
         turn.due = false;
         if (MODE == MCD_MODE_DS) {
-            ch = group_event<T, REC, G>(L, sig, c, cur, active, w.w, g, zmax, use_tab, &ev, &turn);
+            ch = group_event<T, REC, G>(L, sig, c, cur, active, w.w, plain, g, zmax, use_tab, &ev, &turn);
         } else if (active) {
             if (step >= w.w) {
                 lane_long(L);
