@@ -334,10 +334,16 @@ int mcd_run(const mcd_sim* sim, const mcd_material* mat,
  * per group of DS simulations with the same material, Wc and density) that
  * the kernel interpolates instead of evaluating 3 + n_shells formulas per
  * event (tune variant bit 1 keeps the formulas).
- * mcd_run_batched then only resets the queue and launches (the persistent
- * kernel, and after it the one that runs down the electrons still on their way
- * when the queue is empty, which it lists in the workspace), so it can be
+ * mcd_run_batched then only resets the queue and launches, so it can be
  * captured in a CUDA graph.  tallies[nsims] and status are device pointers.
+ * mcd_batch_prepare_list also takes a device buffer in which the persistent
+ * kernel lists the electrons still on their way when the queue is empty, and a
+ * second kernel then runs them down with fuller warps: two to three times
+ * faster where trajectories are uneven and the batch is a few times the launch
+ * or less.  It is scratch of one launch, so batches that never run at the same
+ * time can share one; mcd_batch_list_bytes(electrons of the batch) is what a
+ * batch can use.  Without it (or with one too small) a launch ends as its lanes
+ * fall idle.  Results do not depend on it.
  * Replaces MapScatterer.__call__ (MC/doScatter.py:54-95) with its pool of
  * multiTraj_* jobs.                                                          */
 size_t mcd_batch_workspace_bytes(int32_t nsims);
@@ -349,6 +355,14 @@ int mcd_batch_prepare(const mcd_sim* sims, int32_t nsims,
                       const mcd_table* tables, const int32_t* sim_moller,
                       const int32_t* sim_gryz, void* workspace,
                       size_t workspace_bytes, void* stream);
+size_t mcd_batch_list_bytes(int64_t electrons);
+int mcd_batch_prepare_list(const mcd_sim* sims, int32_t nsims,
+                           const mcd_material* mats,
+                           const int32_t* sim_material,
+                           const mcd_table* tables, const int32_t* sim_moller,
+                           const int32_t* sim_gryz, void* workspace,
+                           size_t workspace_bytes, void* list,
+                           size_t list_bytes, void* stream);
 int mcd_run_batched(void* workspace, int32_t nsims, mcd_tally* tallies,
                     const mcd_tune* tune, uint32_t* status, void* stream);
 

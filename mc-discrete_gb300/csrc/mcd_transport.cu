@@ -70,8 +70,11 @@ struct BatchHeader {
     unsigned long long total;   // electrons over all simulations
     int32_t nsims;
     int32_t chan;               // some simulation counts channels
-    int32_t pad_[8];
+    uint32_t* list;             // the list's seats, or nullptr
+    int32_t list_cap;           // ... how many
+    int32_t pad_[5];
 };
+static_assert(sizeof(BatchHeader) == 64, "the workspace's layout");
 
 constexpr int kBatchMaxSims = 256;
 
@@ -112,15 +115,14 @@ __host__ __device__ constexpr size_t batch_sig_off(int nsims) {
 __host__ __device__ constexpr size_t batch_sig_bytes() {   // one table slot per simulation
     return sizeof(float) * (size_t)kSigRowsMax * kSigStride;
 }
-// | the electrons still on their way when the queue ran empty (seats as in
-// mcd_drain.cuh): at most one per lane of the launch
-constexpr int kLiveSeats = 1 << 18;
-__host__ __device__ constexpr size_t batch_live_off(int nsims) {
+__host__ __device__ constexpr size_t batch_bytes(int nsims) {
     return batch_sig_off(nsims) + batch_sig_bytes() * (size_t)nsims;
 }
-__host__ __device__ constexpr size_t batch_bytes(int nsims) {
-    return batch_live_off(nsims) + sizeof(uint32_t) * kSeatWords * (size_t)kLiveSeats;
-}
+// The electrons still on their way when the queue ran empty are listed (seats
+// as in mcd_drain.cuh) in a buffer of its own, scratch of one launch that
+// batches may share: at most one electron per lane of the launch, and no more
+// than the batch has.
+constexpr int kLiveSeats = 1 << 18;
 
 __host__ __device__ constexpr size_t batch_smem(int nsims) {
     return sizeof(SimConst<float>) * nsims + sizeof(unsigned long long) * (nsims + 1) +
@@ -212,7 +214,7 @@ struct BatchShared {
 };
 
 constexpr int kRunInline = 1;   // evaluate cross sections instead of reading the tables
-constexpr int kRunList = 2;     // list the electrons left when the queue is empty
+constexpr int kRunList = 2;     // list the electrons left when the queue is empty, if the list holds them
 
 template <bool REC, bool CHAN>
 __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, int refill, uint32_t* status,
@@ -222,6 +224,7 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
     const int nsims = hdr->nsims;
     const unsigned long long total = hdr->total;
     const int inline_sigma = flags & kRunInline;
+    if ((unsigned long long)hdr->list_cap < min(total, (unsigned long long)gridDim.x * blockDim.x)) flags &= ~kRunList;
     const BatchShared sh(smem, nsims);
     SimConst<float>* s_c = sh.c;
     unsigned long long* s_pre = sh.pre;
@@ -271,8 +274,7 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
                 if (lane == 0 && busy) at = atomicAdd(&hdr->live, (unsigned long long)__popc(busy));
                 at = __shfl_sync(0xffffffffu, at, 0);
                 if (have)
-                    seat_put(Seats{reinterpret_cast<uint32_t*>(ws + batch_live_off(nsims)), kLiveSeats},
-                             (int)at + __popc(busy & lt), L, rng, sim);
+                    seat_put(Seats{hdr->list, hdr->list_cap}, (int)at + __popc(busy & lt), L, rng, sim);
                 break;
             }
         }
@@ -328,7 +330,7 @@ __global__ void __launch_bounds__(kDrainThreads) k_rundown(uint8_t* ws, mcd_tall
     sh.load(ws, nsims);
     __syncthreads();
     const ManySims run{sh.c, sh.t, tallies, reinterpret_cast<const mcd_electron_out*>(ws + batch_elout_off(nsims))};
-    const Seats list{reinterpret_cast<uint32_t*>(ws + batch_live_off(nsims)), kLiveSeats};
+    const Seats list{hdr->list, hdr->list_cap};
     const unsigned count = (live - blockIdx.x + gridDim.x - 1) / gridDim.x;
     auto take = [&](unsigned k, Lane<float>& L, ElecRng& rng, int& sim) {
         seat_get(list, (int)(blockIdx.x + k * gridDim.x), L, rng, sim);
@@ -678,6 +680,11 @@ extern "C" size_t mcd_batch_workspace_bytes(int32_t nsims) {
     return batch_bytes(nsims);
 }
 
+extern "C" size_t mcd_batch_list_bytes(int64_t electrons) {
+    if (electrons <= 0) return 0;
+    return sizeof(uint32_t) * kSeatWords * (size_t)(electrons < kLiveSeats ? electrons : kLiveSeats);
+}
+
 extern "C" size_t mcd_batch_upload_bytes(int32_t nsims) {
     if (nsims <= 0 || nsims > kBatchMaxSims) return 0;
     return batch_sig_off(nsims);
@@ -686,11 +693,20 @@ extern "C" size_t mcd_batch_upload_bytes(int32_t nsims) {
 extern "C" int mcd_batch_prepare(const mcd_sim* sims, int32_t nsims, const mcd_material* mats,
                                  const int32_t* sim_material, const mcd_table* tables, const int32_t* sim_moller,
                                  const int32_t* sim_gryz, void* workspace, size_t workspace_bytes, void* stream) {
+    return mcd_batch_prepare_list(sims, nsims, mats, sim_material, tables, sim_moller, sim_gryz, workspace,
+                                  workspace_bytes, nullptr, 0, stream);
+}
+
+extern "C" int mcd_batch_prepare_list(const mcd_sim* sims, int32_t nsims, const mcd_material* mats,
+                                      const int32_t* sim_material, const mcd_table* tables,
+                                      const int32_t* sim_moller, const int32_t* sim_gryz, void* workspace,
+                                      size_t workspace_bytes, void* list, size_t list_bytes, void* stream) {
     if (!sims || !mats || !sim_material || !workspace) return MCD_EINVAL;
     if (nsims <= 0) return MCD_EINVAL;
     if (nsims > kBatchMaxSims) return MCD_ETOOBIG;
     if (workspace_bytes < batch_bytes(nsims)) return MCD_EINVAL;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255) != 0) return MCD_EINVAL;
+    if ((reinterpret_cast<uintptr_t>(list) & 3) != 0) return MCD_EINVAL;
     const size_t bytes = batch_sig_off(nsims);   // everything but the tables, which the GPU fills
     uint8_t* host = static_cast<uint8_t*>(calloc(1, bytes));
     if (!host) return MCD_EINVAL;
@@ -729,6 +745,9 @@ extern "C" int mcd_batch_prepare(const mcd_sim* sims, int32_t nsims, const mcd_m
     h->total = acc;
     h->nsims = nsims;
     for (int k = 0; k < nsims; ++k) h->chan |= (sims[k].tally_flags & MCD_TALLY_CHANNELS) ? 1 : 0;
+    const size_t seats = list ? list_bytes / (sizeof(uint32_t) * kSeatWords) : 0;
+    h->list = static_cast<uint32_t*>(list);
+    h->list_cap = (int32_t)(seats < (size_t)kLiveSeats ? seats : (size_t)kLiveSeats);
     if (rc == MCD_OK) {
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         const unsigned grid = (unsigned)(((long long)nsims * kSigRowsMax + 255) / 256);

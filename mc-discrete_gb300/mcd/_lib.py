@@ -224,6 +224,10 @@ SIGNATURES = {
     "mcd_batch_prepare": (C.c_int, [C.POINTER(Sim), C.c_int32, C.POINTER(Material), C.POINTER(C.c_int32),
                                     C.POINTER(Table), C.POINTER(C.c_int32), C.POINTER(C.c_int32),
                                     C.c_void_p, C.c_size_t, C.c_void_p]),
+    "mcd_batch_list_bytes": (C.c_size_t, [C.c_int64]),
+    "mcd_batch_prepare_list": (C.c_int, [C.POINTER(Sim), C.c_int32, C.POINTER(Material), C.POINTER(C.c_int32),
+                                         C.POINTER(Table), C.POINTER(C.c_int32), C.POINTER(C.c_int32),
+                                         C.c_void_p, C.c_size_t, C.c_void_p, C.c_size_t, C.c_void_p]),
     "mcd_run_batched": (C.c_int, [C.c_void_p, C.c_int32, C.c_void_p, C.POINTER(Tune), C.c_void_p,
                                   C.c_void_p]),
     "mcd_run_batched_noalloc": (C.c_int, [C.POINTER(Sim), C.c_int32, C.POINTER(Material), C.POINTER(C.c_int32),

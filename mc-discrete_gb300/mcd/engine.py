@@ -366,16 +366,25 @@ def run(input_par, num_el=None, seed=0, first_electron=0, precision="fp32", elec
 # ---------------------------------------------------------------------------
 # batched persistent launch
 # ---------------------------------------------------------------------------
+def run_down_list(electrons, device="cuda"):
+    """The device buffer in which a batched launch of so many electrons lists
+    the ones still on their way when its queue is empty."""
+    return _torch().empty(_lib.lib().mcd_batch_list_bytes(int(electrons)), dtype=_torch().uint8, device=device)
+
+
 class Batch:
     """Many simulations run by one persistent kernel.
 
     sims: list of input_par dicts (each with num_el).  Tables are built once
     per distinct (material, E0, Emin, Wc, tol) and shared.  electrons=True
-    keeps every simulation's per-electron rows (electrons(k)).
+    keeps every simulation's per-electron rows (electrons(k)).  scratch: the
+    run-down list of a launch (run_down_list), for batches that never run at the
+    same time to share; by default the batch has its own.
     """
 
     def __init__(self, sims, seed=0, device="cuda", hist_E=DEFAULT_HIST_E, hist_T=DEFAULT_HIST_T,
-                 quirks=_lib.QUIRKS_REFERENCE, tally_channels=False, first_electron=0, electrons=False):
+                 quirks=_lib.QUIRKS_REFERENCE, tally_channels=False, first_electron=0, electrons=False,
+                 scratch=None):
         torch = _torch()
         self.device = torch.device(device)
         self.inputs = [with_defaults(s) for s in sims]
@@ -429,19 +438,20 @@ class Batch:
         off = (-self.workspace.data_ptr()) % 256
         self.ws_ptr = self.workspace.data_ptr() + off
         self.ws_bytes = nbytes
+        self.total_electrons = sum(int(p["num_el"]) for p in self.inputs)
+        self.scratch = scratch if scratch is not None else run_down_list(self.total_electrons, self.device)
         self.prepare()
         self.tallies = torch.zeros((self.n, C.sizeof(_lib.Tally)), dtype=torch.uint8, device=self.device)
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
-        self.total_electrons = sum(int(p["num_el"]) for p in self.inputs)
 
     def prepare(self, stream=None):
         """Pack the simulations into the device workspace (host-to-device copy)."""
         torch = _torch()
         st = stream if stream is not None else torch.cuda.current_stream(self.device)
-        code = _lib.lib().mcd_batch_prepare(self._sims_arr, self.n, self.mats, self._idx[0], self._tarr,
-                                            self._idx[1], self._idx[2], self.ws_ptr, self.ws_bytes,
-                                            st.cuda_stream)
-        _lib.check("mcd_batch_prepare", code)
+        code = _lib.lib().mcd_batch_prepare_list(self._sims_arr, self.n, self.mats, self._idx[0], self._tarr,
+                                                 self._idx[1], self._idx[2], self.ws_ptr, self.ws_bytes,
+                                                 self.scratch.data_ptr(), self.scratch.numel(), st.cuda_stream)
+        _lib.check("mcd_batch_prepare_list", code)
 
     def launch(self, tune=None, stream=None):
         torch = _torch()

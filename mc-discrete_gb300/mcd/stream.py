@@ -21,7 +21,7 @@ import time
 
 from . import _lib
 from .config import with_defaults
-from .engine import Batch, _torch, event_dtype
+from .engine import Batch, _torch, event_dtype, run_down_list
 
 
 class EventStream:
@@ -48,13 +48,15 @@ class EventStream:
         self.device = torch.device(device)
         self.tune = tune if tune is not None else _lib.Tune(256, 0, 1, 0, 0)
         self.nchunks = (self.num_el + self.chunk - 1) // self.chunk
-        # one prepared workspace per chunk (built once, so launches never wait on the host)
+        # one prepared workspace per chunk (built once, so launches never wait on
+        # the host); the chunks run one after the other and share a run-down list
         self.batches = []
+        scratch = run_down_list(self.chunk, self.device)
         for c in range(self.nchunks):
             first = c * self.chunk
             n = min(self.chunk, self.num_el - first)
             self.batches.append(Batch([dict(self.p, num_el=n)], seed=self.seed, device=self.device,
-                                      first_electron=first))
+                                      first_electron=first, scratch=scratch))
         epe = events_per_electron or 1000.0
         cap = int(ring_events) if ring_events else int(1.3 * epe * self.chunk) + 4096
         self.piece = max(self.rec_bytes, (int(piece_bytes) // self.rec_bytes) * self.rec_bytes)
