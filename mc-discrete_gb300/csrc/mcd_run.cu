@@ -26,17 +26,17 @@ __global__ void __launch_bounds__(THREADS) k_run(const SimConst<float> cp, const
                                                  mcd_tally* tally, const mcd_electron_out eo,
                                                  const mcd_event_ring ring, uint32_t* status) {
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ BlockTally bt;
+    __shared__ BlockTally bt[THREADS / 32];   // a copy per warp
     __shared__ SimConst<float> c;
     __shared__ mcd_electron_out rows;
     if (threadIdx.x == 0) {
         c = cp;
         rows = eo;
     }
-    bt_zero(&bt, 1);
+    bt_zero(bt, THREADS / 32);
     __syncthreads();
     const HotConst<float> hot(c, MODE == MCD_MODE_CONT ? &keys : nullptr);
-    const OneSim<MODE, HotConst<float>> run{c, hot, bt, tally, rows};
+    const OneSim<MODE, HotConst<float>> run{c, hot, bt[threadIdx.x >> 5], tally, rows};
     const unsigned count = (unsigned)(((unsigned long long)c.num_el - blockIdx.x + gridDim.x - 1) / gridDim.x);
     auto take = [&](unsigned k, Lane<float>& L, ElecRng& rng, int& sim) {
         rng = elec_rng(c, c.first + blockIdx.x + (uint64_t)k * gridDim.x);
@@ -48,7 +48,9 @@ __global__ void __launch_bounds__(THREADS) k_run(const SimConst<float> cp, const
                                                     : drain_run<REC, false>(run, count, take, smem, ring, false);
     or_status(status, st);
     __syncthreads();
-    if (threadIdx.x == 0) bt_flush(bt, tally, chan);
+    bt_fold(bt, 1, THREADS / 32);
+    __syncthreads();
+    if (threadIdx.x == 0) bt_flush(bt[0], tally, chan);
 }
 
 template <int MODE, bool REC>

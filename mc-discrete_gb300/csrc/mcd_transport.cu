@@ -128,8 +128,17 @@ __host__ __device__ constexpr size_t batch_smem(int nsims) {
     return sizeof(SimConst<float>) * nsims + sizeof(unsigned long long) * (nsims + 1) +
            sizeof(int32_t) * ((nsims + 1) & ~1) + sizeof(BlockTally) * nsims;
 }
-// ... of the run-down kernel, the drain's seats after it
-__host__ __device__ constexpr size_t batch_drain_off(int nsims) { return (batch_smem(nsims) + 15) & ~(size_t)15; }
+// Copies of the tallies in the run-down kernel (bt_fold): one for each of its 16
+// warps while they take no more than 17 KB.
+__host__ __device__ constexpr int drain_copies(int nsims) {
+    int c = kDrainThreads / 32;
+    while (c > 1 && c * nsims > 80) c /= 2;
+    return c;
+}
+// Its shared memory: that of the batch, the other copies, the drain's seats.
+__host__ __device__ constexpr size_t batch_drain_off(int nsims) {
+    return (batch_smem(nsims) + sizeof(BlockTally) * nsims * (drain_copies(nsims) - 1) + 15) & ~(size_t)15;
+}
 
 // Queue order: simulations with the longest expected trajectories first, so
 // that the last electrons handed out are short ones and the grid drains
@@ -196,7 +205,7 @@ struct BatchShared {
           pre(reinterpret_cast<unsigned long long*>(smem + sizeof(SimConst<float>) * nsims)),
           perm(reinterpret_cast<int32_t*>(pre + (nsims + 1))),
           t(reinterpret_cast<BlockTally*>(perm + ((nsims + 1) & ~1))) {}
-    __device__ __forceinline__ void load(const uint8_t* ws, int nsims) const {
+    __device__ __forceinline__ void load(const uint8_t* ws, int nsims, int copies = 1) const {
         const uint32_t* src = reinterpret_cast<const uint32_t*>(ws + batch_consts_off(nsims));
         uint32_t* dst = reinterpret_cast<uint32_t*>(c);
         const int words = (int)(sizeof(SimConst<float>) / 4) * nsims;
@@ -205,7 +214,7 @@ struct BatchShared {
         for (int k = threadIdx.x; k <= nsims; k += blockDim.x) pre[k] = p[k];
         const int32_t* q = reinterpret_cast<const int32_t*>(ws + batch_perm_off(nsims));
         for (int k = threadIdx.x; k < nsims; k += blockDim.x) perm[k] = q[k];
-        bt_zero(t, nsims);
+        bt_zero(t, nsims * copies);
     }
     __device__ __forceinline__ void flush(mcd_tally* tallies, int nsims) const {
         for (int k = threadIdx.x; k < nsims; k += blockDim.x)
@@ -327,9 +336,11 @@ __global__ void __launch_bounds__(kDrainThreads) k_rundown(uint8_t* ws, mcd_tall
     const unsigned live = (unsigned)hdr->live;
     if (blockIdx.x >= live) return;
     const BatchShared sh(smem, nsims);
-    sh.load(ws, nsims);
+    const int copies = drain_copies(nsims);
+    sh.load(ws, nsims, copies);
     __syncthreads();
-    const ManySims run{sh.c, sh.t, tallies, reinterpret_cast<const mcd_electron_out*>(ws + batch_elout_off(nsims))};
+    BlockTally* mine = sh.t + (int)(threadIdx.x >> 5) % copies * nsims;
+    const ManySims run{sh.c, mine, tallies, reinterpret_cast<const mcd_electron_out*>(ws + batch_elout_off(nsims))};
     const Seats list{hdr->list, hdr->list_cap};
     const unsigned count = (live - blockIdx.x + gridDim.x - 1) / gridDim.x;
     auto take = [&](unsigned k, Lane<float>& L, ElecRng& rng, int& sim) {
@@ -340,7 +351,7 @@ __global__ void __launch_bounds__(kDrainThreads) k_rundown(uint8_t* ws, mcd_tall
     uint32_t st;
     if (ONE && !(sh.c[0].bits & kBitCont)) {
         const HotConst<float> hot(sh.c[0]);
-        const OneSim<MCD_MODE_DS, HotConst<float>> one{sh.c[0], hot, sh.t[0], tallies, run.rows(0)};
+        const OneSim<MCD_MODE_DS, HotConst<float>> one{sh.c[0], hot, mine[0], tallies, run.rows(0)};
         st = hdr->chan ? drain_run<REC, true>(one, count, take, seats, ring, inl)
                        : drain_run<REC, false>(one, count, take, seats, ring, inl);
     } else {
@@ -348,6 +359,8 @@ __global__ void __launch_bounds__(kDrainThreads) k_rundown(uint8_t* ws, mcd_tall
                        : drain_run<REC, false>(run, count, take, seats, ring, inl);
     }
     or_status(status, st);
+    __syncthreads();
+    bt_fold(sh.t, nsims, copies);
     __syncthreads();
     sh.flush(tallies, nsims);
 }
