@@ -30,9 +30,15 @@ namespace mcd {
 // itself made nvcc 13.0 (sm_103a, -O3) drop the loop-carried energy update of
 // the lane state initialised from it; the shared-memory copy is also what the
 // batched kernel reads.
+// The continuous model keeps the constants in registers and reads the round keys
+// from the constant bank (RoundKeys): its events are short, and a run of a warp or
+// two per scheduler waits for each load and addition on the way to the random
+// words.  6080 electrons of Au 30 keV 0.675 -> 0.579 ms, of Al 0.266 -> 0.231, 36480 of
+// Cu 0.446 -> 0.398, 1e6 of Al 5 keV 0.917 -> 0.891.
 template <class T, int MODE, bool REC>
-__global__ void __launch_bounds__(256) k_plain(const SimConst<T> cp, mcd_tally* tally, const ElOut eo,
-                                               const mcd_event_ring ring, uint32_t* status) {
+__global__ void __launch_bounds__(256) k_plain(const SimConst<T> cp, const __grid_constant__ RoundKeys keys,
+                                               mcd_tally* tally, const ElOut eo, const mcd_event_ring ring,
+                                               uint32_t* status) {
     __shared__ BlockTally bt;
     __shared__ SimConst<T> c;
     if (threadIdx.x == 0) c = cp;
@@ -45,10 +51,11 @@ __global__ void __launch_bounds__(256) k_plain(const SimConst<T> cp, mcd_tally* 
         lane_init(L, c);
         const ElecRng rng = elec_rng(c, c.first + i);
         const bool chan = (c.tally_flags & MCD_TALLY_CHANNELS) != 0;
+        const HotConst<T> hot(c, MODE == MCD_MODE_CONT ? &keys : nullptr);   // (continuous)
         while (L.outcome == MCD_OUT_NONE) {
             EventOut<T> ev;
             const int ch = (MODE == MCD_MODE_DS) ? ds_event<T, REC>(L, c, rng, &ev, c.sig != nullptr)
-                                                 : cont_event<T, REC>(L, c, rng, &ev);
+                                                 : cont_event<T, REC>(L, hot, rng, &ev);
             if (ch >= 0) {
                 if (REC) st |= ring_append(ring, (uint32_t)i, L.step, ev);
                 if (chan && ch != MCD_CH_RUTH) atomicAdd(&bt.channel[ch], 1ull);
@@ -523,7 +530,7 @@ static int launch_plain(const SimConst<T>& c, int block, mcd_tally* tally, const
     const unsigned long long grid = ((unsigned long long)c.num_el + block - 1) / block;
     if (grid == 0) return MCD_OK;
     if (grid > 0x7fffffffull) return MCD_ETOOBIG;
-    k_plain<T, MODE, REC><<<(unsigned)grid, block, 0, st>>>(c, tally, eo, ring, status);
+    k_plain<T, MODE, REC><<<(unsigned)grid, block, 0, st>>>(c, round_keys(c), tally, eo, ring, status);
     return cudaGetLastError() == cudaSuccess ? MCD_OK : MCD_ECUDA;
 }
 
