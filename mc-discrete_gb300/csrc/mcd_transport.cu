@@ -54,12 +54,16 @@ __global__ void __launch_bounds__(256) k_plain(const SimConst<T> cp, const __gri
         const HotConst<T> hot(c, MODE == MCD_MODE_CONT ? &keys : nullptr);   // (continuous)
         while (L.outcome == MCD_OUT_NONE) {
             EventOut<T> ev;
+            RingTicket tk{};
+            if (REC) {
+                const bool rec = L.step < c.max_scatt, takes = ring_takes(ring, (uint32_t)i);
+                tk = ring_reserve(ring, rec && takes);
+                if (rec && !takes) st |= MCD_FLAG_RING_INDEX;
+            }
             const int ch = (MODE == MCD_MODE_DS) ? ds_event<T, REC>(L, c, rng, &ev, c.sig != nullptr)
                                                  : cont_event<T, REC>(L, hot, rng, &ev);
-            if (ch >= 0) {
-                if (REC) st |= ring_append(ring, (uint32_t)i, L.step, ev);
-                if (chan && ch != MCD_CH_RUTH) atomicAdd(&bt.channel[ch], 1ull);
-            }
+            if (REC) ring_write(ring, ring_slot(ring, tk), (uint32_t)i, L.step, ev);
+            if (chan && ch > MCD_CH_RUTH) atomicAdd(&bt.channel[ch], 1ull);
         }
         st |= finish_electron(c, L, i, bt, tally, eo);
     }
