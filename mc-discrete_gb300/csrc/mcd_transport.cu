@@ -560,8 +560,10 @@ static int dispatch_plain(const SimConst<T>& c, int block, mcd_tally* tally, con
 //   (Au: 3500 1.07 / 1.26 with 32 / 16, 4500 1.35 / 1.34 with 16 / 8, 7500
 //   1.53 / 1.63 with 8 / 0, 10000 1.83 / 1.72; Cu without a table: 3500 0.88 /
 //   0.85, 4500 0.95 / 1.08, 7500 1.21 / 1.23, 10000 1.36 / 1.32)
-//   FP32 continuous      1500: 0.21 / 0.23 with 32 / 8;  2500: 0.28 / 0.24;
-//                        4500: 0.25 / 0.27 with 8 / 0;  6500: 0.28 / 0.28
+//   FP32 continuous (44 parameter sets of all materials, 32 / 8 lanes over 0, the
+//                        mean and the worst): 10 per SM 0.91, 0.95 / 0.97, 0.99; 14:
+//                        1.02, 1.13 / 0.97, 0.98;  18: 1.15, 1.33 / 1.01, 1.06; 33:
+//                        1.54, 2.08 / 1.08, 1.19
 //   FP64 DS (with their host calls; Si, table)  1200: 2.15 / 2.31 with 32 / 16,
 //                        1400: 2.63 / 2.37;  2100: 2.60 / 2.82 with 16 / 8, 2500:
 //                        3.76 / 3.10 (up to two warps per scheduler, both);
@@ -577,7 +579,7 @@ static int dispatch_plain(const SimConst<T>& c, int block, mcd_tally* tally, con
 static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) {
     const int64_t e = s.num_el / sms;   // electrons per SM
     if (s.precision == MCD_FP32) {
-        if (s.mode != MCD_MODE_DS) return e < 12 ? 32 : e < 34 ? 8 : 0;
+        if (s.mode != MCD_MODE_DS) return e < 12 ? 32 : e < 16 ? 8 : 0;
         return e < 20 ? 32 : e < 33 ? 16 : e < 58 ? 8 : 0;
     }
     if (s.mode != MCD_MODE_DS) return e < 3 ? 32 : e < 18 ? 8 : 0;
@@ -593,17 +595,37 @@ static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) 
 //   FP32 DS    always (10000 electrons: Cu 1.32 / 1.96, Au 1.72 / 2.74, Si 0.59
 //              / 0.75; 80000: Cu 2.23 / 2.66, Au 3.16 / 4.01, Si 0.88 / 0.98;
 //              1e6: Cu 12.6 / 21.5, Au 12.9 / 33.4, Si 5.7 / 8.0)
-//   FP32 continuous, whose lengths differ by backscattering alone: 1e6
-//              electrons Cu 70 deg 2.50 / 4.26, Al 70 deg 1.77 / 2.27, Au 0 deg
-//              7.5 / 10.8, Cu 0 deg 3.97 / 4.30, but Al 0 deg 2.39 / 2.28;
-//              (Cu 70 deg 100000: 0.48 / 0.58, 40000: 0.33 / 0.36, 10000: 0.28
-//              / 0.28)
+//   FP32 continuous, whose lengths differ by backscattering alone: only where
+//              they differ much (tilted beams, heavy elements) and the run is
+//              large; up to 1024 electrons per SM the independent threads are all
+//              resident at once.  The line moves up as trajectories get shorter,
+//              as the ends weigh more.  Time over that of independent threads:
+//                electrons per SM      300   400   600   800  1000  1300  2500  5000
+//                Al  5 keV 60 deg     1.20  1.16  1.09  1.01  1.01  1.03  0.96  0.91
+//                Al  5 keV 75 deg     1.24  1.16  1.08  1.02  0.97  0.86  0.85  0.78
+//                Al 10 keV 60 deg     1.17  1.07  1.02  0.94  0.99  1.02  0.92  0.87
+//                Al 30 keV 60 deg     1.09  1.00  0.93  0.84  0.92  0.96  0.87  0.82
+//                Al 30 keV  0 deg     1.17  1.01  1.01  0.92  1.26  1.19  1.07  0.99
+//                Cu  5 keV 60 deg     1.16  1.07  1.00  0.89  0.93  0.82  0.82  0.74
+//                Cu 30 keV 60 deg     1.06  0.92  0.84  0.73  0.76  0.74  0.69  0.67
+//                Cu 30 keV  0 deg     1.08  0.98  0.92  0.81  1.10  0.95  0.94  0.86
+//                Au  5 keV  0 deg     1.11  0.96  0.89  0.77  0.78  0.74  0.76  0.68
+//                Au 30 keV  0 deg     1.04  0.88  0.81  0.69  0.73  0.73  0.68  0.66
+//                Au 30 keV 75 deg     0.93  0.77  0.71  0.56  0.56  0.48  0.40  0.37
+//              (500: within 0.1 above 400; films of 1000 A, in which light elements
+//              and fast beams make short trajectories: Al 10 keV 60 deg 500: 1.18,
+//              1000: 1.06, 2500: 0.80; Cu 30 keV 75 deg 1.13, 1.15, 0.81; Cu 10 keV
+//              80 deg 0.98, 0.70, 0.47)
 static bool one_block_per_sm(const mcd_sim& s, const mcd_material& m, int sms) {
     const int64_t e = s.num_el / sms;   // electrons per SM
     if (s.precision != MCD_FP32 || e > INT32_MAX / 2) return false;
     if (s.mode == MCD_MODE_DS) return true;
     if (s.E0 < 10.0 * s.Emin) return false;   // short trajectories: the start and the end weigh more
-    if (s.s_tilt >= 60.0 || m.Z >= 40) return e >= 230;
+    const bool film = s.thickness > 0 && s.thickness < 1e30;
+    if (film && (m.Z < 25 || s.E0 > 15e3) && e <= 1024) return false;
+    if (m.Z >= 40) return e >= (s.E0 >= 10e3 || s.s_tilt >= 60.0 ? 400 : 600);
+    if (s.s_tilt >= 60.0 && m.Z >= 25) return e >= (s.E0 >= 20e3 ? 400 : 600);
+    if (s.s_tilt >= 60.0) return e >= (s.E0 >= 8e3 ? 800 : 1300);
     return m.Z >= 25 && e >= 4000;
 }
 
