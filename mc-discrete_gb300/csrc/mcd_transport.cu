@@ -595,6 +595,10 @@ static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) 
 //   FP32 DS    always (10000 electrons: Cu 1.32 / 1.96, Au 1.72 / 2.74, Si 0.59
 //              / 0.75; 80000: Cu 2.23 / 2.66, Au 3.16 / 4.01, Si 0.88 / 0.98;
 //              1e6: Cu 12.6 / 21.5, Au 12.9 / 33.4, Si 5.7 / 8.0)
+//              but for the thinnest films, of an event or two, while the independent
+//              threads are all resident at once (30 A at 5 keV, 300 to 1000 electrons
+//              per SM: 1.0 to 1.14 of their time; 100 A at 15 keV 0.9 to 1.16; 100 A at
+//              5 keV 0.5 to 1.1, at 30 keV 0.96 to 1.14)
 //   FP32 continuous, whose lengths differ by backscattering alone: only where
 //              they differ much (tilted beams, heavy elements) and the run is
 //              large; up to 1024 electrons per SM the independent threads are all
@@ -619,9 +623,9 @@ static int lanes_per_electron(const mcd_sim& s, const mcd_material& m, int sms) 
 static bool one_block_per_sm(const mcd_sim& s, const mcd_material& m, int sms) {
     const int64_t e = s.num_el / sms;   // electrons per SM
     if (s.precision != MCD_FP32 || e > INT32_MAX / 2) return false;
-    if (s.mode == MCD_MODE_DS) return true;
-    if (s.E0 < 10.0 * s.Emin) return false;   // short trajectories: the start and the end weigh more
     const bool film = s.thickness > 0 && s.thickness < 1e30;
+    if (s.mode == MCD_MODE_DS) return !(film && s.thickness < 0.007 * s.E0 && e <= 1024);
+    if (s.E0 < 10.0 * s.Emin) return false;   // short trajectories: the start and the end weigh more
     if (film && (m.Z < 25 || s.E0 > 15e3) && e <= 1024) return false;
     if (m.Z >= 40) return e >= (s.E0 >= 10e3 || s.s_tilt >= 60.0 ? 400 : 600);
     if (s.s_tilt >= 60.0 && m.Z >= 25) return e >= (s.E0 >= 20e3 ? 400 : 600);
