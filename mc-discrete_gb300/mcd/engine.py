@@ -125,7 +125,11 @@ _TALLY_WORDS = [(f[0], getattr(_lib.Tally, f[0]).offset // 8, getattr(_lib.Tally
 
 def tally_from_bytes(buf):
     """An mcd_tally's bytes as a dict."""
-    w = np.frombuffer(bytes(buf), dtype=np.int64)
+    size = C.sizeof(_lib.Tally)
+    raw = bytes(buf)[:size]
+    if len(raw) < size:
+        raise ValueError("an mcd_tally has %d bytes, not %d" % (size, len(raw)))
+    w = np.frombuffer(raw, dtype=np.int64)
     f = {k: w[a:a + n] for k, a, n in _TALLY_WORDS}
     out = {k: int(f["outcome"][i]) for i, k in enumerate(_lib.OUTCOME_NAMES)}
     for k in ("events", "double_rows", "nan_events", "clamped", "long_path", "table_range"):
