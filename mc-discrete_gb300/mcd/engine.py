@@ -155,8 +155,9 @@ class _Store:
     copies, one per array, took about as long as its transport.
 
     add(dtype, n) reserves an array and returns its number, make(device)
-    allocates, self[k] is array k on the device, and host() reads everything
-    back once and returns k -> array k in host memory."""
+    allocates, self[k] is array k on the device, and host(size) reads the first
+    `size` bytes (None: everything) back once and returns k -> array k in that
+    one host buffer."""
 
     def __init__(self):
         self.spans, self.size = [], 0
@@ -175,19 +176,22 @@ class _Store:
     def __getitem__(self, k):
         return self.arrays[k]
 
-    def host(self):
-        b = self.bytes.cpu()
+    def host(self, size=None):
+        b = self.bytes[:size].cpu()
         return lambda k: b[self.spans[k][1]:self.spans[k][1] + self.spans[k][2]].view(self.spans[k][0]).numpy()
 
 
 _ROWS = ("outcome", "flags", "final_E", "dir", "last_pos", "max_z", "n_events")
+_PLANES = ("dir", "last_pos")
 
 
 def _add_rows(store, n, fdt):
-    """Reserves the per-electron row arrays (the mcd_electron_out layout)."""
+    """Reserves the per-electron row arrays (mcd_electron_out's), the planes last."""
     torch = _torch()
-    kinds = ((torch.uint8, n), (torch.uint8, n), (fdt, n), (fdt, 3 * n), (fdt, 3 * n), (fdt, n), (torch.int32, n))
-    return {k: store.add(dt, m) for k, (dt, m) in zip(_ROWS, kinds)}
+    at = {k: store.add(dt, n) for k, dt in (("outcome", torch.uint8), ("flags", torch.uint8), ("final_E", fdt),
+                                            ("max_z", fdt), ("n_events", torch.int32))}
+    at.update({k: store.add(fdt, 3 * n) for k in _PLANES})
+    return {k: at[k] for k in _ROWS}
 
 
 def _rows_struct(e):
@@ -197,15 +201,32 @@ def _rows_struct(e):
 
 
 _DEVICE_TRANSPOSE = 8192   # electrons from which the device turns the planes (100000: 15 us against 320 in NumPy)
+# ... and from which every array has a copy over the link of its own, as the host
+# copies out of one buffer cost more (100000: a read-back of 310 us with them, 255
+# without; 20000: 210 and 240).
+_ROWS_APART = 65536
+
+
+def _read_rows(store, rows, n):
+    """The one copy to the host of a run's arrays, without those that are read by
+    themselves (_Store.host)."""
+    if not rows or n < _DEVICE_TRANSPOSE:
+        return store.host()
+    return store.host(store.spans[rows["dir" if n < _ROWS_APART else "outcome"]][1])
 
 
 def _host_rows(el, n, host):
-    """Per-electron rows on the host (dir and last_pos as (n, 3)); el: the
-    device arrays, host(name): their copies on the host."""
-    e = {k: host(k) for k in _ROWS if n < _DEVICE_TRANSPOSE or k not in ("dir", "last_pos")}
-    for k in ("dir", "last_pos"):
-        e[k] = e[k].reshape(3, n).T.copy() if k in e else el[k].view(3, n).t().contiguous().cpu().numpy()
-    return {k: e[k] for k in ("outcome", "flags", "final_E", "dir", "last_pos", "max_z", "n_events")}
+    """Per-electron rows on the host, each an array of its own (dir and last_pos
+    as (n, 3)); el: the device arrays, host(name): their copies in the one
+    buffer."""
+    def row(k):
+        if k not in _PLANES:
+            return host(k).copy() if n < _ROWS_APART else el[k].cpu().numpy()
+        if n < _DEVICE_TRANSPOSE:
+            return host(k).reshape(3, n).T.copy()
+        return el[k].view(3, n).t().contiguous().cpu().numpy()
+
+    return {k: row(k) for k in _ROWS}
 
 
 class RunBuffers:
@@ -328,7 +349,7 @@ def launch(sim, mat, tables, bufs, block_size=0, stream=None):
 
 def collect(bufs):
     """Copy the results of the last launch back to the host (synchronises)."""
-    host = bufs._store.host()
+    host = _read_rows(bufs._store, bufs._rows, bufs.num_el)
     k_tally, k_status, k_cursor = bufs._read
     tally = tally_from_bytes(host(k_tally))
     status = int(host(k_status)[0])
@@ -506,6 +527,7 @@ class Batch:
         """Simulation k's per-electron rows on the host (electrons=True)."""
         if self.el is None:
             raise RuntimeError("the batch keeps no per-electron rows (electrons=False)")
+        n = int(self.inputs[k]["num_el"])
         st, rows = self._el_stores[k]
-        host = st.host()
-        return _host_rows(self.el[k], int(self.inputs[k]["num_el"]), lambda name: host(rows[name]))
+        host = _read_rows(st, rows, n)
+        return _host_rows(self.el[k], n, lambda name: host(rows[name]))
