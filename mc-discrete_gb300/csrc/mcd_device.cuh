@@ -1147,16 +1147,6 @@ __device__ __forceinline__ void ring_write(const mcd_event_ring& ring, unsigned 
     }
 }
 
-// Both at once, for the lanes that call it together.
-template <class T>
-__device__ __forceinline__ uint32_t ring_append(const mcd_event_ring& ring, uint32_t electron, uint32_t step,
-                                                const EventOut<T>& ev) {
-    const bool takes = ring_takes(ring, electron);
-    const RingTicket k = ring_reserve(ring, takes);
-    ring_write(ring, ring_slot(ring, k), electron, step, ev);
-    return takes ? 0u : MCD_FLAG_RING_INDEX;
-}
-
 // Lets a kernel be launched with `bytes` of dynamic shared memory.  What a block
 // has without asking for more is 48 KB less the kernel's static arrays (the
 // run-down kernel has some 500 bytes); a kernel that needs more is allowed all

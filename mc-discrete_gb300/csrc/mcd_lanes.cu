@@ -94,6 +94,12 @@ __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst
         }
         const EventPre<T> next = pre[((step + 1) / G) & 1][g.h0 + (int)((step + 1) & (G - 1))];
         EventOut<T> ev;
+        RingTicket tk{};
+        if (REC) {
+            const bool rec = g.t == 0 && active && step < w.w, takes = ring_takes(ring, (uint32_t)i);
+            tk = ring_reserve(ring, rec && takes);
+            if (rec && !takes) st |= MCD_FLAG_RING_INDEX;
+        }
         int ch = kGroupNone;
         turn.due = false;
         if (MODE == MCD_MODE_DS) {
@@ -113,7 +119,7 @@ __global__ void __launch_bounds__(32, lanes_blocks<T>(G)) k_lanes(const SimConst
             if (G < 32) __syncwarp();
             group_turn<G>(L, turn, cur.cph, cur.sph, g);
         }
-        if (REC && g.t == 0 && ch != kGroupNone) st |= ring_append(ring, (uint32_t)i, L.step, ev);
+        if (REC) ring_write(ring, ring_slot(ring, tk), (uint32_t)i, L.step, ev);
         if (ch != kGroupPlain && active) {
             if (g.t == 0 && chan && ch > MCD_CH_RUTH) atomicAdd(&bt.channel[ch], 1ull);
             if (L.outcome != MCD_OUT_NONE) {
