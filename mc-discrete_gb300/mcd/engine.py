@@ -201,10 +201,11 @@ def _rows_struct(e):
 
 
 _DEVICE_TRANSPOSE = 8192   # electrons from which the device turns the planes (100000: 15 us against 320 in NumPy)
-# ... and from which every array has a copy over the link of its own, as the host
-# copies out of one buffer cost more (100000: a read-back of 310 us with them, 255
-# without; 20000: 210 and 240).
-_ROWS_APART = 65536
+# ... and from which every array is read back by itself.  In between the columns
+# stay in the buffer that one copy brought, a few MB at most, without the planes:
+# taking them out costs more than reading them did (100000: 27 us to read, 98 to
+# take out, 89 to read one by one).
+_ROWS_APART = 1 << 18
 
 
 def _read_rows(store, rows, n):
@@ -216,15 +217,15 @@ def _read_rows(store, rows, n):
 
 
 def _host_rows(el, n, host):
-    """Per-electron rows on the host, each an array of its own (dir and last_pos
-    as (n, 3)); el: the device arrays, host(name): their copies in the one
-    buffer."""
+    """Per-electron rows on the host, each an array of its own (but for the middle
+    sizes' columns), dir and last_pos as (n, 3); el: the device arrays,
+    host(name): their copies in the one buffer."""
     def row(k):
-        if k not in _PLANES:
-            return host(k).copy() if n < _ROWS_APART else el[k].cpu().numpy()
         if n < _DEVICE_TRANSPOSE:
-            return host(k).reshape(3, n).T.copy()
-        return el[k].view(3, n).t().contiguous().cpu().numpy()
+            return (host(k).reshape(3, n).T if k in _PLANES else host(k)).copy()
+        if k in _PLANES:
+            return el[k].view(3, n).t().contiguous().cpu().numpy()
+        return host(k) if n < _ROWS_APART else el[k].cpu().numpy()
 
     return {k: row(k) for k in _ROWS}
 

@@ -39,19 +39,23 @@ def collected(n):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [0, 1, 1000, 8191, 8192, 65535, 65536, 100003])
-def test_rows_are_arrays_of_their_own(n):
+@pytest.mark.parametrize("n", [0, 1, 1000, 8191, 8192, 100003, 2 ** 18 - 1, 2 ** 18])
+def test_rows_hold_no_more_than_they_need(n):
     bufs, rows = collected(n)
     want = np.arange(3 * n, dtype=np.float32).reshape(3, n).T
     assert np.array_equal(rows["dir"], want) and np.array_equal(rows["last_pos"], want + 1)
     assert np.array_equal(rows["n_events"], np.arange(n))
     assert list(rows) == ["outcome", "flags", "final_E", "dir", "last_pos", "max_z", "n_events"]
+    # the columns of the middle sizes share a buffer that holds nothing larger
+    columns = sum(a.nbytes for k, a in rows.items() if k not in ("dir", "last_pos")) + C.sizeof(_lib.Tally) + 8 * 512
     for k, a in rows.items():
-        assert a.flags.writeable and a.flags.c_contiguous and held_bytes(a) == a.nbytes, k
+        own = k in ("dir", "last_pos") or not 8192 <= n < 2 ** 18
+        assert a.flags.writeable and a.flags.c_contiguous, k
+        assert held_bytes(a) == a.nbytes if own else held_bytes(a) <= columns, k
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [50000, 100000])
+@pytest.mark.parametrize("n", [50000, 300000])
 def test_large_rows_cross_the_link_once(monkeypatch, n):
     import torch
     crossed = []
