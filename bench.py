@@ -51,15 +51,15 @@ CPU_SAMPLE_ELECTRONS = 40000
 # of a smaller launch of the same simulations: tables and workspace read about
 # once, and the run-down kernel's list; the figure does not grow with the
 # electrons
-BATCHED_DRAM_BYTES = 54.46e6 + 2.39e6 + 19.41e6
+BATCHED_DRAM_BYTES = 54.42e6 + 1.52e6 + 19.51e6
 # warp instructions issued per event by both kernels on this workload in its
 # tuned shape (two blocks of 576 per SM, 56 registers), from that capture
-# (2.167e10 and 6.99e8 instructions for 1.7539e9 events); the issue peak is one
+# (2.148e10 and 7.01e8 instructions for 1.7539e9 events); the issue peak is one
 # warp instruction per scheduler per cycle, 4 schedulers per SM
-WARP_INST_PER_EVENT = 12.75
+WARP_INST_PER_EVENT = 12.65
 # the same capture's fractions of the persistent kernel: issue-active cycles,
 # threads per warp instruction / 32, the L1/TEX unit
-BATCHED_NCU = {"issue_active": 0.757, "warp_execution_efficiency": 0.775, "l1tex_throughput": 0.84,
+BATCHED_NCU = {"issue_active": 0.762, "warp_execution_efficiency": 0.75, "l1tex_throughput": 0.82,
                "capture": "ncu counters of k_batched_lr (2 x 576, 56 registers) on the 64 simulations with "
                           "10^U[2.5, 5.5] electrons (1.7539e9 events)"}
 

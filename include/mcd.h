@@ -338,9 +338,9 @@ int mcd_run(const mcd_sim* sim, const mcd_material* mat,
  * captured in a CUDA graph.  tallies[nsims] and status are device pointers.
  * mcd_batch_prepare_list also takes a device buffer in which the persistent
  * kernel lists the electrons still on their way when the queue is empty, and a
- * second kernel then runs them down with fuller warps: two to three times
- * faster where trajectories are uneven and the batch is a few times the launch
- * or less.  It is scratch of one launch, so batches that never run at the same
+ * second kernel then runs them down with fuller warps (six uneven simulations
+ * 7.8 -> 4.6 ms, 40000 Au electrons 5.8 -> 4.0, 1e6 16.6 -> 14.6; a batch of a
+ * few short trajectories pays some 5 us).  It is scratch of one launch, so batches that never run at the same
  * time can share one; mcd_batch_list_bytes(electrons of the batch) is what a
  * batch can use.  Without it (or with one too small) a launch ends as its lanes
  * fall idle.  Results do not depend on it.

@@ -180,10 +180,10 @@ __device__ __forceinline__ void batched_body(uint8_t* ws, mcd_tally* tallies, in
 
 // Two register budgets of the same kernel: up to 1024 threads per block at
 // 64 registers (32 warps per SM: one block of 1024), or two blocks of up to
-// 576 per SM at 56 registers (36 warps, 8 bytes spilled, two copies of the
-// constant blocks in shared memory): on the 64-simulation workload the
-// second, in blocks of 576, is 1.2% faster (78.2 against 79.1 ms); five
-// blocks of 256 at 48 registers were 26% slower.
+// 576 per SM at 56 registers (36 warps, two copies of the constant blocks in
+// shared memory); neither spills.  On the 64-simulation workload the second, in
+// blocks of 576, takes 72.4 ms against 74.2; five blocks of 256 at 48 registers
+// were 26% slower.
 // REC: append every event to the ring.  The event loop exists twice, CHAN
 // for batches in which some simulation counts channels, so that the others
 // test nothing per event (one test there cost 1% of the 64 simulations); the
